@@ -159,6 +159,7 @@ int check_status(eimp_ctx *ctx) {
         if (st & EIMP_ERR_BEAM_EMPTY) return fail(ctx, EIMP_E_BEAM_EMPTY, "Beam is empty. No paths left.");
         if (st & EIMP_ERR_QREF_TRUNCATED) return fail(ctx, EIMP_E_ARG, "Truncated runlength sequence!");
         if (st & EIMP_ERR_HAPLOID_HET) return fail(ctx, EIMP_E_ARG, "Found heterozygous genotype in haploid target.");
+        if (st & EIMP_ERR_WAIT) return fail(ctx, EIMP_E_CUDA, "a kernel's wait for its own copies ran out");
         char b[160];
         snprintf(b, sizeof b, "device structure capacity exceeded (status 0x%x)", st);
         return fail(ctx, EIMP_E_CAPACITY, b);
@@ -353,7 +354,7 @@ int eimp_imp_set_reference_dev(eimp_ctx *ctx, size_t Mref, size_t nhaps, const u
     CK(ctx->i_segm.reserve(Mref * 4));
     CK(ctx->i_common.reserve(Mref));
     CK(ctx->i_sinfo.reserve(Mref * sizeof(int2)));
-    CK(ctx->i_compr.reserve(M * kw * 4));
+    CK(ctx->i_compr.reserve(M * kw * 4 + 16));   // the match search copies whole 16-byte pieces
     CK(ctx->i_absperm.reserve((M + 1) * K * 4));
     CK(ctx->i_count0.reserve(M * 4));
     CK(cudaMemcpyAsync(ctx->i_af.p, d_af_full, Mref * 4, cudaMemcpyDeviceToDevice, st));

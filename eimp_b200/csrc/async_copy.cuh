@@ -1,0 +1,51 @@
+// Bulk copies from global to shared memory that complete on an mbarrier
+// (cp.async.bulk), with bounded waits.
+#pragma once
+
+#include <cstdint>
+#include <cuda_runtime.h>
+
+namespace eimp {
+
+// Polls after which a wait gives up.  A poll (mbarrier.try_wait) suspends the
+// thread for a hardware-chosen time of at most a few microseconds, so the limit
+// is seconds -- far beyond any copy -- and a kernel whose barrier is never
+// completed still ends.
+constexpr int MBAR_POLLS = 1 << 20;
+
+__device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void mbar_init(uint64_t *bar, int arrivals) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(arrivals) : "memory");
+}
+// makes the initialised barriers visible to the copy engine
+__device__ __forceinline__ void mbar_init_fence() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
+    asm volatile("{ .reg .b64 t; mbarrier.arrive.shared::cta.b64 t, [%0]; }" ::"r"(smem_addr(bar)) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(uint64_t *bar, unsigned bytes) {
+    asm volatile("{ .reg .b64 t; mbarrier.arrive.expect_tx.shared::cta.b64 t, [%0], %1; }" ::"r"(smem_addr(bar)),
+                 "r"(bytes)
+                 : "memory");
+}
+// waits for the phase with the given parity; false when it gave up
+__device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity) {
+    for (int i = 0; i < MBAR_POLLS; i++) {
+        unsigned done;
+        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                     : "=r"(done)
+                     : "r"(smem_addr(bar)), "r"(parity)
+                     : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+// bytes (a multiple of 16) from global src to shared dst, both 16-byte aligned
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, unsigned bytes, uint64_t *bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_addr(dst)),
+                 "l"(src), "r"(bytes), "r"(smem_addr(bar))
+                 : "memory");
+}
+
+}  // namespace eimp

@@ -8,7 +8,9 @@
 //                      haplotype: the rank queries of all tree nodes of a
 //                      site and the rebuild of the tree run across the lanes;
 //                      the compact kernel stores the tree in 30 B per node
-//                      (typed sites < 65536).
+//                      (typed sites < 65536).  Without set-maximal errors the
+//                      first launch is smm_list_kernel (smm_list.cu), and
+//                      these kernels only retry what outgrows its lists.
 //  dosage_kernel    -- TargetImp::imputeBunch (TargetImp.cpp:474-558), one
 //                      warp per (target haplotype, span of 64-site tiles).
 #include <climits>
@@ -1165,7 +1167,10 @@ static cudaError_t smm_launch(Kern kern, int warps, const uint32_t *compr, const
 }
 
 size_t smm_gpool_slot_bytes(int K) {
-    return K <= 65536 ? sizeof(SmmWarpSmemC<SMM_NODES_RETRY, uint16_t>) : sizeof(SmmWarpSmemC<SMM_NODES_RETRY, int>);
+    const size_t tree =
+        K <= 65536 ? sizeof(SmmWarpSmemC<SMM_NODES_RETRY, uint16_t>) : sizeof(SmmWarpSmemC<SMM_NODES_RETRY, int>);
+    const size_t list = smm_list_slot_bytes(K);
+    return tree > list ? tree : list;
 }
 
 template <typename IV>
@@ -1178,8 +1183,13 @@ static cudaError_t launch_smm_compact(const uint32_t *compr, const int32_t *coun
     using Big = SmmWarpSmemC<SMM_NODES_RETRY, IV>;
     Big *gp = static_cast<Big *>(gpool);
     cudaError_t e;
-    // warps per CTA of the first pass: 1, 2 or 4
-    if (warps == 1)
+    // without set-maximal errors the list kernel searches (2.8 to 4.3 times
+    // as fast at every size measured); otherwise warps per CTA of the first
+    // pass: 1, 2 or 4
+    if (setmaxerrors <= 0)
+        e = launch_smm_list(compr, M, K, phased, wM, gt, nhaps, hapmap, matches, cap, nmatch, status, gpool,
+                            gpool_slots, gpool_next, st);
+    else if (warps == 1)
         e = smm_launch<Small>(smm_compact_kernel<SMM_NODES, 1, false, IV>, 1, compr, count0, M, K, phased, wM, gt,
                               nhaps, hapmap, setmaxerrors, matches, cap, nmatch, status, st, gp, gpool_slots,
                               gpool_next);
@@ -1209,9 +1219,12 @@ cudaError_t launch_smm(const uint32_t *compr, const int32_t *count0, int M, int 
         return launch_smm_compact<int>(compr, count0, M, K, phased, wM, gt, nhaps, hapmap, setmaxerrors, matches, cap,
                                        nmatch, status, warps, gpool, gpool_slots, gpool_next, st);
     }
-    cudaError_t e = smm_launch<SmmWarpSmem<SMM_NODES>>(smm_kernel<SMM_NODES, SMM_WARPS, false>, SMM_WARPS, compr,
-                                                       count0, M, K, phased, wM, gt, nhaps, hapmap, setmaxerrors,
-                                                       matches, cap, nmatch, status, st);
+    cudaError_t e = setmaxerrors <= 0
+                        ? launch_smm_list(compr, M, K, phased, wM, gt, nhaps, hapmap, matches, cap, nmatch, status,
+                                          gpool, gpool_slots, gpool_next, st)
+                        : smm_launch<SmmWarpSmem<SMM_NODES>>(smm_kernel<SMM_NODES, SMM_WARPS, false>, SMM_WARPS, compr,
+                                                             count0, M, K, phased, wM, gt, nhaps, hapmap, setmaxerrors,
+                                                             matches, cap, nmatch, status, st);
     if (e != cudaSuccess) return e;
     return smm_launch<SmmWarpSmem<SMM_NODES_RETRY>>(smm_kernel<SMM_NODES_RETRY, 1, true>, 1, compr, count0, M, K,
                                                     phased, wM, gt, nhaps, hapmap, setmaxerrors, matches, cap, nmatch,

@@ -47,6 +47,13 @@ cudaError_t launch_smm(const uint32_t *compr, const int32_t *count0, int M, int 
                        int *nmatch, uint32_t *status, int warps, void *gpool, int gpool_slots, int *gpool_next,
                        cudaStream_t st);
 size_t smm_gpool_slot_bytes(int K);
+// the first launch of the match search without set-maximal errors
+// (smm_list.cu); compr is readable up to the next 16-byte boundary past its
+// end.  Haplotypes it marks are redone by launch_smm's retry launch.
+cudaError_t launch_smm_list(const uint32_t *compr, int M, int K, const uint64_t *phased, int wM, const uint8_t *gt,
+                            int nhaps, const int32_t *hapmap, int4 *matches, int cap, int *nmatch, uint32_t *status,
+                            void *gpool, int gpool_slots, int *gpool_next, cudaStream_t st);
+size_t smm_list_slot_bytes(int K);
 // refmap (null: identity): panel haplotype of each PBWT haplotype (the
 // reduced reference without the haploid samples' placeholder columns)
 cudaError_t launch_dosage(const int4 *matches, int cap, const int *nmatch, const int32_t *absperm, int K,
