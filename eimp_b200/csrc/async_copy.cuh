@@ -1,5 +1,6 @@
-// Bulk copies from global to shared memory that complete on an mbarrier
-// (cp.async.bulk), with bounded waits.
+// Asynchronous copies from global to shared memory: bulk copies that complete
+// on an mbarrier (cp.async.bulk), with bounded waits, and per-thread copies in
+// groups (cp.async).
 #pragma once
 
 #include <cstdint>
@@ -46,6 +47,28 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src, unsigned b
                      smem_addr(dst)),
                  "l"(src), "r"(bytes), "r"(smem_addr(bar))
                  : "memory");
+}
+
+
+// 16 or 8 bytes by the calling thread, both addresses aligned to the size
+__device__ __forceinline__ void copy_async16(void *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async8(void *dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+// closes the calling thread's group of copies
+__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// waits until at most N of the calling thread's groups are in flight
+template <int N> __device__ __forceinline__ void copy_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// a barrier of 'threads' threads of the CTA, reached from any place in the code
+__device__ __forceinline__ void block_barrier(int threads) { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); }
+// further ones, by number
+__device__ __forceinline__ void pair_barrier(int k, int threads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + k), "r"(threads) : "memory");
 }
 
 }  // namespace eimp

@@ -12,8 +12,12 @@
 #define SMMC_WARPS 2
 #define SMM_NODES 512
 #define SMM_NODES_RETRY 4096
-// beam phasing: warps (targets) per CTA
+// beam phasing: warps per target where an SM holds several targets (at most
+// BEAM_SM_CTAS) and where it holds one
 #define BEAM_WARPS 4
+#define BEAM_MAX_WARPS 8
+#define BEAM_SM_CTAS 3
+#define BEAM_RECORDS 128   // haplotype-path records in shared memory, at most
 
 namespace eimp {
 
@@ -143,10 +147,10 @@ struct BeamParams {
     const uint8_t *startph = nullptr;
 };
 size_t beam_arena_bytes(const BeamParams &p, int S_max);
-// warps of the persistent beam launch for ntgt targets (a multiple of the
-// warps per CTA; at most the resident ones), -1 on a CUDA error
+// CTAs of the persistent beam launch for ntgt targets (pct % of the resident
+// ones), -1 on a CUDA error
 int beam_slots(const BeamParams &p, int M, int ntgt, int pct = 100);
-// the persistent beam: slots warps (beam_slots), one arena of arena_bytes per
+// the persistent beam: slots CTAs (beam_slots), one arena of arena_bytes per
 // slot; order (ntgt ints) and workq (one int) are scratch: the longest-first
 // order and the queue counter, both filled here
 cudaError_t launch_beam(const BeamParams &p, int ntgt, int M, const uint8_t *gt, const uint64_t *monos,

@@ -29,4 +29,18 @@ inline void bulk_load(void *dst, const void *src, unsigned bytes, uint64_t *b) {
     memcpy(dst, src, bytes);
     mbar_arrive(b);
 }
+inline void emu_copy(void *dst, const void *src, size_t n) {
+    if (((uintptr_t)dst | (uintptr_t)src) & (n - 1)) { fprintf(stderr, "asynchronous copy off %zu bytes\n", n); abort(); }
+    memcpy(dst, src, n);
+}
+inline void copy_async16(void *dst, const void *src) { emu_copy(dst, src, 16); }
+inline void copy_async8(void *dst, const void *src) { emu_copy(dst, src, 8); }
+inline void copy_async_commit() {}
+template <int N> inline void copy_async_wait() {}
+inline void block_barrier(int) { emu_block->arrive_and_wait(); }
+inline void pair_barrier(int k, int threads) {   // among warps of the same block
+    static EmuBarrier bars[4];
+    bars[k].n = threads;
+    bars[k].arrive_and_wait();
+}
 }  // namespace eimp
