@@ -359,7 +359,6 @@ int eimp_imp_set_reference_dev(eimp_ctx *ctx, size_t Mref, size_t nhaps, const u
     CK(ctx->i_count0.reserve(M * 4));
     CK(cudaMemcpyAsync(ctx->i_af.p, d_af_full, Mref * 4, cudaMemcpyDeviceToDevice, st));
     CK(cudaMemcpyAsync(ctx->i_typed.p, d_typed, M * 8, cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemsetAsync(ctx->i_hapfull.p, 0, nhaps * wMref * 8, st));
     LAUNCH(launch_transpose(d_sitemajor_full, Mref, wN, ctx->i_hapfull.as<uint64_t>(), nhaps, wMref, st));
     LAUNCH(launch_segmap(ctx->i_typed.as<int64_t>(), (int)M, (int)Mref, ctx->i_af.as<float>(), (int)nhaps,
                          ctx->i_segm.as<int32_t>(), ctx->i_common.as<uint8_t>(), ctx->i_sinfo.as<int2>(), st));
@@ -378,7 +377,7 @@ int eimp_imp_set_reference_dev(eimp_ctx *ctx, size_t Mref, size_t nhaps, const u
                                    ctx->i_sitetyped_c.as<uint64_t>(), (int)wK, st));
         typed_rows = ctx->i_sitetyped_c.as<uint64_t>();
     }
-    const size_t rps = refpbwt_scratch_bytes((int)K, (int)wK);
+    const size_t rps = refpbwt_scratch_bytes((int)M, (int)K, (int)wK);
     if (rps) CK(ctx->i_rpscratch.reserve(rps));
     LAUNCH(launch_refpbwt(typed_rows, (int)M, (int)K, (int)wK, ctx->i_compr.as<uint32_t>(),
                           ctx->i_absperm.as<int32_t>(), ctx->i_count0.as<int32_t>(),
@@ -944,7 +943,6 @@ int eimp_phase_set_reference_dev(eimp_ctx *ctx, size_t M, size_t nhaps, const ui
     CK(ctx->p_cm.reserve(M * 4));
     LAUNCH(launch_gather_rows(d_sitemajor_full, ldw_words, d_typed, (int)M, (int)wN, ctx->p_sitemajor.as<uint64_t>(),
                               st));
-    CK(cudaMemsetAsync(ctx->p_hapmajor.p, 0, nhaps * wM * 8, st));
     LAUNCH(launch_transpose(ctx->p_sitemajor.as<uint64_t>(), M, wN, ctx->p_hapmajor.as<uint64_t>(), nhaps, wM, st));
     CK(cudaMemcpyAsync(ctx->p_cm.p, d_cM, M * 4, cudaMemcpyDeviceToDevice, st));
     return 0;
@@ -1254,7 +1252,6 @@ int eimp_gpu_initialize(eimp_ctx *ctx, size_t K, size_t Kwords, size_t M, size_t
     // haplotype-major copy for the condensed-reference kernel
     const size_t wM = eimp_W(M);
     CK(ctx->g_hapT.reserve(NrefhapsAD * wM * 8));
-    CK(cudaMemsetAsync(ctx->g_hapT.p, 0, NrefhapsAD * wM * 8, ctx->stream));
     LAUNCH(launch_transpose(ctx->g_refT.as<uint64_t>(), M, refTCapacity / 8, ctx->g_hapT.as<uint64_t>(), NrefhapsAD,
                             wM, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));

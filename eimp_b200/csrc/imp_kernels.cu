@@ -67,6 +67,7 @@ __device__ void block_exscan(int *a, int n, int *warpbuf, int *total) {
 // compressed row and zero count of its interval.
 // ---------------------------------------------------------------------------
 constexpr int RP_CK = 64;     // sites between checkpoint orders
+constexpr int RP_SUB = 16;    // sites between the orders of refpbwt_blocks.cu
 constexpr int RP_BITS = 5;    // sites per step of the checkpoint pass: 32 buckets, one per lane
 // rounds of 32 positions whose loads are issued together: 8 with the orders
 // in global memory (their latency overlapped), 1 in shared memory (fewer
@@ -200,16 +201,18 @@ __global__ void __launch_bounds__(1024, 1) refpbwt_ckpt_kernel(const uint64_t *_
     }
 }
 
-// Fill pass: CTA c covers sites [c*RP_CK, min(M, (c+1)*RP_CK)); the order
-// before its first site is the checkpoint.  Per site: the bits in prefix
+// Fill pass: CTA c covers sites [c*CK, min(M, (c+1)*CK)); the order before its
+// first site is there (from the checkpoint pass, or every RB_SUB sites from
+// refpbwt_blocks.cu).  Per site: the bits in prefix
 // order (one ballot per 32 positions), the zeros per 32-position word and
 // their exclusive scan give the compressed row [data, cumulative zeros] and
-// the stable partition into the next order (PBWT.cpp:207-285).
-__global__ void __launch_bounds__(1024) refpbwt_fill_kernel(const uint64_t *__restrict__ sitemajor, int M, int K,
-                                                           int wN, uint32_t *__restrict__ compr,
-                                                           int32_t *__restrict__ absperm,
-                                                           int32_t *__restrict__ count0) {
-    extern __shared__ uint8_t smem[];
+// the stable partition into the next order (PBWT.cpp:207-285).  FU: words whose
+// part of the order a warp loads before it uses any (one at a time the loads'
+// latency is what a site of a large panel takes).
+template <int CK, int FU>
+__device__ __forceinline__ void fill_sites(uint8_t *smem, const uint64_t *__restrict__ sitemajor, int M, int K, int wN,
+                                           uint32_t *__restrict__ compr, int32_t *__restrict__ absperm,
+                                           int32_t *__restrict__ count0) {
     const int nwords = (K + 31) / 32;
     uint32_t *row = reinterpret_cast<uint32_t *>(smem);                  // 2*wN u32
     uint32_t *data = row + 2 * wN;                                       // nwords
@@ -218,7 +221,7 @@ __global__ void __launch_bounds__(1024) refpbwt_fill_kernel(const uint64_t *__re
     int *tot = warpbuf + 32;                                             // 1
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nwarps = blockDim.x >> 5;
     const size_t kw = 2 * (size_t)nwords;
-    const int m0 = blockIdx.x * RP_CK, m1 = min(M, m0 + RP_CK);
+    const int m0 = blockIdx.x * CK, m1 = min(M, m0 + CK);
 
     for (int m = m0; m < m1; m++) {
         const uint64_t *src = sitemajor + (size_t)m * wN;
@@ -230,37 +233,50 @@ __global__ void __launch_bounds__(1024) refpbwt_fill_kernel(const uint64_t *__re
         __syncthreads();
         const int32_t *perm = absperm + (size_t)m * K;
         int32_t *nperm = absperm + (size_t)(m + 1) * K;
-        // the order before the next checkpoint site exists already
-        const bool put = !((m + 1) % RP_CK == 0 && m + 1 < M);
+        // the order before the next CTA's first site exists already
+        const bool put = !((m + 1) % CK == 0 && m + 1 < M);
         // pass 1: bits in prefix order, zeros per 32-position word
-        for (int w = wid; w < nwords; w += nwarps) {
-            int i = w * 32 + lane;
-            int bit = 1;
-            if (i < K) {
-                int h = perm[i];
-                bit = (row[h >> 5] >> (h & 31)) & 1;
+        for (int w0 = wid; w0 < nwords; w0 += FU * nwarps) {
+            int h[FU];
+#pragma unroll
+            for (int u = 0; u < FU; u++) {
+                const int i = (w0 + u * nwarps) * 32 + lane;
+                h[u] = i < K ? perm[i] : -1;
             }
-            uint32_t b = __ballot_sync(0xffffffffu, bit);
-            if (lane == 0) { data[w] = b; pz[w] = __popc(~b); }
+#pragma unroll
+            for (int u = 0; u < FU; u++) {
+                const int w = w0 + u * nwarps;
+                const int bit = h[u] >= 0 ? (row[h[u] >> 5] >> (h[u] & 31)) & 1 : 1;
+                const uint32_t b = __ballot_sync(0xffffffffu, bit);
+                if (lane == 0 && w < nwords) { data[w] = b; pz[w] = __popc(~b); }
+            }
         }
         __syncthreads();
         block_exscan(pz, nwords, warpbuf, tot);
         const int cnt0 = *tot;
         // pass 2: scatter into the next order, emit compressed words
         uint32_t *crow = compr + (size_t)m * kw;
-        for (int w = wid; w < nwords; w += nwarps) {
-            int i = w * 32 + lane;
-            uint32_t b = data[w];
-            int zb = pz[w];
-            if (i < K && put) {
-                int h = perm[i];
-                uint32_t lt = (1u << lane) - 1u;
-                int dst = ((b >> lane) & 1) ? cnt0 + (w * 32 - zb) + __popc(b & lt) : zb + __popc(~b & lt);
-                nperm[dst] = h;
+        for (int w0 = wid; w0 < nwords; w0 += FU * nwarps) {
+            int h[FU];
+#pragma unroll
+            for (int u = 0; u < FU; u++) {
+                const int i = (w0 + u * nwarps) * 32 + lane;
+                h[u] = i < K && put ? perm[i] : -1;
             }
-            if (lane == 0) {
-                crow[2 * w] = b;
-                crow[2 * w + 1] = (uint32_t)(zb + __popc(~b));
+#pragma unroll
+            for (int u = 0; u < FU; u++) {
+                const int w = w0 + u * nwarps;
+                if (w >= nwords) continue;
+                const uint32_t b = data[w];
+                const int zb = pz[w];
+                if (h[u] >= 0) {
+                    const uint32_t lt = (1u << lane) - 1u;
+                    nperm[((b >> lane) & 1) ? cnt0 + (w * 32 - zb) + __popc(b & lt) : zb + __popc(~b & lt)] = h[u];
+                }
+                if (lane == 0) {
+                    crow[2 * w] = b;
+                    crow[2 * w + 1] = (uint32_t)(zb + __popc(~b));
+                }
             }
         }
         if (tid == 0) count0[m] = cnt0;
@@ -268,27 +284,96 @@ __global__ void __launch_bounds__(1024) refpbwt_fill_kernel(const uint64_t *__re
     }
 }
 
+__global__ void __launch_bounds__(1024) refpbwt_fill_kernel(const uint64_t *__restrict__ sitemajor, int M, int K,
+                                                           int wN, uint32_t *__restrict__ compr,
+                                                           int32_t *__restrict__ absperm,
+                                                           int32_t *__restrict__ count0) {
+    extern __shared__ uint8_t smem[];
+    fill_sites<RP_CK, 1>(smem, sitemajor, M, K, wN, compr, absperm, count0);
+}
+
+// the same from the orders of refpbwt_blocks.cu
+template <int FU>
+__global__ void __launch_bounds__(1024) refpbwt_fill_sub_kernel(const uint64_t *__restrict__ sitemajor, int M, int K,
+                                                                int wN, uint32_t *__restrict__ compr,
+                                                                int32_t *__restrict__ absperm,
+                                                                int32_t *__restrict__ count0) {
+    extern __shared__ uint8_t smem[];
+    fill_sites<RP_SUB, FU>(smem, sitemajor, M, K, wN, compr, absperm, count0);
+}
+
 // ---------------------------------------------------------------------------
 // bit-matrix transpose: src (rows of src_ld words, 'cols' valid bits per row)
-// -> dst (cols rows of dst_ld words, of which the first dstw are written:
-// word w of dst row c holds bit c of src rows 64w .. 64w+63).  One 64x64 tile
-// per block of 64 threads; grid (ceil(rows/64), ceil(cols/64)).
+// -> word w of dst row c holds bit c of src rows 64w .. 64w+63, for the
+// first dstw words of each of the cols dst rows (zeros past the last src row).
+// dst row c starts at c * dst_ld, or -- BLOCKS -- word w of dst row c lies at
+// w * dst_ld + c (the 64 bits of a block of rows, haplotype after haplotype).
+//
+// A CTA takes 256 rows x 16 words: a lane reads the 128 bytes of its row, each
+// 32 x 32 bits are transposed in a warp by five butterfly exchanges, and the
+// 1024 columns are written as 32 bytes each, which neighbouring CTAs complete to
+// lines in L2.  Memory-bound: source and result cross DRAM once.
 // ---------------------------------------------------------------------------
-__global__ void transpose_kernel(const uint64_t *__restrict__ src, size_t rows, size_t src_ld,
-                                 uint64_t *__restrict__ dst, size_t cols, size_t dstw, size_t dst_ld) {
-    __shared__ uint64_t tile[64];
-    const size_t rw = blockIdx.x;      // 64-row block (source rows -> dest word)
-    const size_t cw = blockIdx.y;      // source word (-> 64 dest rows)
-    const int t = threadIdx.x;
-    size_t r = rw * 64 + t;
-    tile[t] = r < rows ? src[r * src_ld + cw] : 0ull;
+constexpr int TR_ROWS = 256, TR_WORDS = 16;   // rows and source words of a tile
+constexpr int TR_LD = TR_ROWS / 32 + 1;       // 32-bit words of a column of the tile, one to skew the banks
+constexpr size_t TR_SMEM = sizeof(uint32_t) * TR_WORDS * 64 * TR_LD;
+
+// bit c of lane r -> bit r of lane c: at distance o a lane keeps half of its bits and
+// takes the others from its partner's word rotated by o (left for the lower
+// lane, right for the upper; no kept bit wraps)
+__device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        const uint32_t m = o == 16 ? 0x0000ffffu : o == 8 ? 0x00ff00ffu : o == 4 ? 0x0f0f0f0fu : o == 2 ? 0x33333333u
+                                                                                                     : 0x55555555u;
+        const uint32_t keep = lane & o ? ~m : m;
+        const uint32_t y = __shfl_xor_sync(0xffffffffu, x, o);
+        x = (x & keep) | (__funnelshift_r(y, y, lane & o ? o : 32 - o) & ~keep);
+    }
+    return x;
+}
+
+template <bool BLOCKS>
+__global__ void __launch_bounds__(TR_ROWS) transpose_kernel(const uint64_t *__restrict__ src, size_t rows, size_t src_ld,
+                                                            uint64_t *__restrict__ dst, size_t cols, size_t dstw,
+                                                            size_t dst_ld) {
+    extern __shared__ uint32_t tr_smem[];
+    uint32_t *tile = tr_smem;   // [column][row / 32]
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const size_t r = (size_t)blockIdx.x * TR_ROWS + t;
+    const size_t cw = (size_t)blockIdx.y * TR_WORDS, ncw = (cols + 63) / 64;
+    const uint64_t *from = src + r * src_ld + cw;
+    // 16 bytes at a time where the rows are aligned and the tile is whole
+    const bool wide = (reinterpret_cast<uintptr_t>(src) & 15) == 0 && (src_ld & 1) == 0 && cw + TR_WORDS <= ncw;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {   // half a tile at a time: the row's words in registers
+        if (cw + h * TR_WORDS / 2 >= ncw) break;
+        uint64_t x[TR_WORDS / 2];
+#pragma unroll
+        for (int k = 0; k < TR_WORDS / 2; k += 2) {
+            const int q = h * TR_WORDS / 2 + k;
+            if (wide) {
+                const uint4 v = r < rows ? *reinterpret_cast<const uint4 *>(from + q) : make_uint4(0u, 0u, 0u, 0u);
+                x[k] = v.x | (uint64_t)v.y << 32;
+                x[k + 1] = v.z | (uint64_t)v.w << 32;
+            } else {
+                x[k] = r < rows && cw + q < ncw ? from[q] : 0ull;
+                x[k + 1] = r < rows && cw + q + 1 < ncw ? from[q + 1] : 0ull;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < TR_WORDS; k++)
+            tile[(32 * (h * TR_WORDS + k) + lane) * TR_LD + warp] =
+                transpose32((uint32_t)(x[k >> 1] >> (32 * (k & 1))), lane);
+    }
     __syncthreads();
-    size_t c = cw * 64 + t;
-    if (c < cols && rw < dstw) {
-        uint64_t o = 0;
-#pragma unroll 8
-        for (int j = 0; j < 64; j++) o |= ((tile[j] >> t) & 1ull) << j;
-        dst[c * dst_ld + rw] = o;
+    const size_t w0 = (size_t)blockIdx.x * (TR_ROWS / 64), c0 = cw * 64;
+    const int nc = cols - c0 < (size_t)TR_WORDS * 64 ? (int)(cols - c0) : TR_WORDS * 64;   // columns of the tile
+    for (int i = t; i < nc * (TR_ROWS / 64); i += TR_ROWS) {
+        const int c = BLOCKS ? i % nc : i / (TR_ROWS / 64), w = BLOCKS ? i / nc : i % (TR_ROWS / 64);
+        if (w0 + w < dstw)
+            dst[BLOCKS ? (w0 + w) * dst_ld + c0 + c : (c0 + c) * dst_ld + w0 + w] =
+                (uint64_t)tile[c * TR_LD + 2 * w] | (uint64_t)tile[c * TR_LD + 2 * w + 1] << 32;
     }
 }
 
@@ -1103,29 +1188,37 @@ static int optin_smem() {
     return v;
 }
 
-size_t refpbwt_scratch_bytes(int K, int wN) {
+size_t refpbwt_scratch_bytes(int M, int K, int wN) {
+    if (refpbwt_by_blocks(M, K)) return 0;
     const size_t lim = (size_t)optin_smem();
     return refpbwt_ckpt_smem(K, wN, true, true) <= lim ? 0 : (size_t)K * 9;
 }
 
 cudaError_t launch_refpbwt(const uint64_t *sitemajor, int M, int K, int wN, uint32_t *compr, int32_t *absperm,
                            int32_t *count0, int32_t *scratch, cudaStream_t st) {
-    const size_t lim = (size_t)optin_smem();
-    const bool in_smem = refpbwt_ckpt_smem(K, wN, true, true) <= lim;
-    if (!in_smem && !scratch) return cudaErrorInvalidValue;
-    const bool stage = refpbwt_ckpt_smem(K, wN, true, in_smem) <= lim;
-    size_t sm = refpbwt_ckpt_smem(K, wN, stage, in_smem);
-    auto ck = in_smem ? refpbwt_ckpt_kernel<1> : refpbwt_ckpt_kernel<8>;
-    cudaError_t e = ensure_dynamic_smem((const void *)ck, sm);
-    if (e != cudaSuccess) return e;
-    ck<<<1, 1024, sm, st>>>(sitemajor, M, K, wN, absperm, in_smem ? nullptr : scratch, stage ? 1 : 0);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    cudaError_t e;
+    if (refpbwt_by_blocks(M, K)) {
+        if ((e = launch_refpbwt_blocks(sitemajor, M, K, wN, absperm, st)) != cudaSuccess) return e;
+    } else {
+        const size_t lim = (size_t)optin_smem();
+        const bool in_smem = refpbwt_ckpt_smem(K, wN, true, true) <= lim;
+        if (!in_smem && !scratch) return cudaErrorInvalidValue;
+        const bool stage = refpbwt_ckpt_smem(K, wN, true, in_smem) <= lim;
+        const size_t sm = refpbwt_ckpt_smem(K, wN, stage, in_smem);
+        auto ck = in_smem ? refpbwt_ckpt_kernel<1> : refpbwt_ckpt_kernel<8>;
+        if ((e = ensure_dynamic_smem((const void *)ck, sm)) != cudaSuccess) return e;
+        ck<<<1, 1024, sm, st>>>(sitemajor, M, K, wN, absperm, in_smem ? nullptr : scratch, stage ? 1 : 0);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
     if (M <= 0) return cudaSuccess;
-    sm = refpbwt_fill_smem(K, wN);
-    if ((e = ensure_dynamic_smem((const void *)refpbwt_fill_kernel, sm)) !=
-        cudaSuccess)
-        return e;
-    refpbwt_fill_kernel<<<(M + RP_CK - 1) / RP_CK, 1024, sm, st>>>(sitemajor, M, K, wN, compr, absperm, count0);
+    const size_t sm = refpbwt_fill_smem(K, wN);
+    // four words a round where every warp has that many (16,384 haplotypes)
+    auto fill = !refpbwt_by_blocks(M, K) ? refpbwt_fill_kernel
+                : K >= 4 * 32 * 32 * 4   ? refpbwt_fill_sub_kernel<4>
+                                         : refpbwt_fill_sub_kernel<1>;
+    const int ck = refpbwt_by_blocks(M, K) ? RP_SUB : RP_CK;
+    if ((e = ensure_dynamic_smem((const void *)fill, sm)) != cudaSuccess) return e;
+    fill<<<(M + ck - 1) / ck, 1024, sm, st>>>(sitemajor, M, K, wN, compr, absperm, count0);
     return cudaGetLastError();
 }
 
@@ -1145,10 +1238,22 @@ cudaError_t launch_transpose(const uint64_t *src, size_t rows, size_t srcw, uint
 cudaError_t launch_transpose_ld(const uint64_t *src, size_t rows, size_t src_ld, uint64_t *dst, size_t cols,
                                 size_t dstw, size_t dst_ld, cudaStream_t st) {
     if (!rows || !cols) return cudaSuccess;
-    const size_t gy = (cols + 63) / 64;
-    if (gy > 65535 || gy > src_ld) return cudaErrorInvalidValue;
-    dim3 grid((unsigned)((rows + 63) / 64), (unsigned)gy);
-    transpose_kernel<<<grid, 64, 0, st>>>(src, rows, src_ld, dst, cols, dstw, dst_ld);
+    const size_t ncw = (cols + 63) / 64, gy = (ncw + TR_WORDS - 1) / TR_WORDS;
+    if (ncw > 65535 || ncw > src_ld) return cudaErrorInvalidValue;
+    cudaError_t e = ensure_dynamic_smem((const void *)transpose_kernel<false>, TR_SMEM);
+    if (e != cudaSuccess) return e;
+    dim3 grid((unsigned)((dstw * 64 + TR_ROWS - 1) / TR_ROWS), (unsigned)gy);
+    transpose_kernel<false><<<grid, TR_ROWS, TR_SMEM, st>>>(src, rows, src_ld, dst, cols, dstw, dst_ld);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_block_keys(const uint64_t *src, int rows, int src_ld, uint64_t *dst, int cols, size_t dst_ld,
+                              cudaStream_t st) {
+    cudaError_t e = ensure_dynamic_smem((const void *)transpose_kernel<true>, TR_SMEM);
+    if (e != cudaSuccess) return e;
+    const int ncw = (cols + 63) / 64;
+    dim3 grid((unsigned)((rows + TR_ROWS - 1) / TR_ROWS), (unsigned)((ncw + TR_WORDS - 1) / TR_WORDS));
+    transpose_kernel<true><<<grid, TR_ROWS, TR_SMEM, st>>>(src, rows, src_ld, dst, cols, (rows + 63) / 64, dst_ld);
     return cudaGetLastError();
 }
 

@@ -29,10 +29,17 @@ cudaError_t ensure_dynamic_smem(const void *kernel, size_t bytes);
 
 
 // ---- imputation (imp_kernels.cu)
-// global scratch launch_refpbwt needs (0: none) for K haplotypes
-size_t refpbwt_scratch_bytes(int K, int wN);
+// global scratch launch_refpbwt needs (0: none) for M sites of K haplotypes
+size_t refpbwt_scratch_bytes(int M, int K, int wN);
 cudaError_t launch_refpbwt(const uint64_t *sitemajor, int M, int K, int wN, uint32_t *compr, int32_t *absperm,
                            int32_t *count0, int32_t *scratch, cudaStream_t st);
+// the checkpoint orders by blocks of 64 sites (refpbwt_blocks.cu) and where they are used
+bool refpbwt_by_blocks(int M, int K);
+cudaError_t launch_refpbwt_blocks(const uint64_t *sitemajor, int M, int K, int wN, int32_t *absperm, cudaStream_t st);
+// word b * dst_ld + c of dst = bits of column c in src rows 64b .. 64b+63 (rows a multiple of 64)
+cudaError_t launch_block_keys(const uint64_t *src, int rows, int src_ld, uint64_t *dst, int cols, size_t dst_ld,
+                              cudaStream_t st);
+// dst row c (dstw words) = column c of the bit matrix src, zeros past its last row
 cudaError_t launch_transpose(const uint64_t *src, size_t rows, size_t srcw, uint64_t *dst, size_t cols, size_t dstw,
                              cudaStream_t st);
 // the same with separate row strides; dstw words of each dst row are written
