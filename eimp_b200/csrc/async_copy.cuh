@@ -29,16 +29,19 @@ __device__ __forceinline__ void mbar_expect(uint64_t *bar, unsigned bytes) {
                  "r"(bytes)
                  : "memory");
 }
-// waits for the phase with the given parity; false when it gave up
+// one poll for the phase with the given parity: true when it is complete
+__device__ __forceinline__ bool mbar_try(uint64_t *bar, unsigned parity) {
+    unsigned done;
+    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                 : "=r"(done)
+                 : "r"(smem_addr(bar)), "r"(parity)
+                 : "memory");
+    return done != 0;
+}
+// waits for it; false when it gave up
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity) {
-    for (int i = 0; i < MBAR_POLLS; i++) {
-        unsigned done;
-        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-                     : "=r"(done)
-                     : "r"(smem_addr(bar)), "r"(parity)
-                     : "memory");
-        if (done) return true;
-    }
+    for (int i = 0; i < MBAR_POLLS; i++)
+        if (mbar_try(bar, parity)) return true;
     return false;
 }
 // bytes (a multiple of 16) from global src to shared dst, both 16-byte aligned

@@ -41,7 +41,7 @@ def emu_exe(tmp_path_factory):
     return str(exe)
 
 
-def run(exe, d, compr, phased, gt, K, wide, warps, group, slots=0, cap=None, hapmap=None):
+def run(exe, d, compr, phased, gt, K, wide, warps, group, slots=0, cap=None, hapmap=None, chunks=1):
     nrows, M = phased.shape[0], gt.shape[1]
     cap = cap or M + 64
     nh = nrows if hapmap is None else len(hapmap)
@@ -51,7 +51,7 @@ def run(exe, d, compr, phased, gt, K, wide, warps, group, slots=0, cap=None, hap
                     ("gt", gt.astype(np.uint8)),
                     ("hapmap", np.asarray([0] if hapmap is None else hapmap, np.int32))]:
         np.ascontiguousarray(a).tofile(os.path.join(d, name + ".bin"))
-    r = subprocess.run([exe, str(d), str(int(wide)), str(warps), str(group), str(slots)], capture_output=True,
+    r = subprocess.run([exe, str(d), str(int(wide)), str(warps), str(group), str(slots), str(chunks)], capture_output=True,
                        text=True, timeout=900)
     assert r.returncode == 0, f"rc {r.returncode}: {r.stderr[-4000:]}"
     m = np.fromfile(os.path.join(d, "o_matches.bin"), np.int32).reshape(nrows, cap, 4).astype(np.int64)
@@ -146,6 +146,63 @@ def test_match_buffer_too_small(emu_exe, tmp_path):
     compr, _, _ = R.pbwt(sm, K)
     _, n, status, _ = run(emu_exe, tmp_path / "k", compr, pack_rows(th, W(M)), gt, K, 0, 8, 4, cap=2)
     assert status == 1 and (n == -1).all()
+
+
+@pytest.mark.parametrize("K,M,wide,warps,group,chunks,err", [(64, 7, 0, 1, 1, 2, 0.0), (300, 150, 0, 3, 4, 3, 0.01),
+                                                             (700, 203, 0, 8, 3, 13, 0.003), (700, 203, 1, 2, 0, 32, 0.01),
+                                                             (500, 320, 0, 5, 16, 10, 0.0), (500, 96, 1, 4, 0, 3, 0.0)])
+def test_chunks_against_oracle(emu_exe, tmp_path, K, M, wide, warps, group, chunks, err):
+    """A haplotype's sites in parts: matches across one and several of their
+    boundaries, one over all sites (a copy of a panel haplotype), parts
+    without a match of their own, sites missing at and around a boundary."""
+    from oracle import restate as R
+    rng = np.random.default_rng(K * 31 + M + chunks)
+    sm, th = panel(rng, M, K, 12, err)
+    th[0] = (sm.reshape(M, -1)[:, 5 // 64] >> np.uint64(5)) & np.uint64(1)
+    gt = np.where(rng.random((4, M)) < 0.06, 3, th[0::2] + th[1::2]).astype(np.uint8)
+    gt[1, M // chunks - 1:M // chunks + 2] = 3
+    gt[3, rng.permutation(M)[:M // 2 + 1]] = 3
+    ph = pack_rows(th, W(M))
+    compr, c0, _ = R.pbwt(sm, K)
+    hapmap = [0, 3, 2, 4, 7]
+    m, n, status, _ = run(emu_exe, tmp_path / "k", compr, ph, gt, K, wide, warps, group, hapmap=hapmap, chunks=chunks,
+                          cap=chunks * (M + 2))
+    assert status == 0
+    for h in hapmap:
+        om = R.smmatches(compr, c0, M, K, ph[h], np.flatnonzero(gt[h // 2] == 3).astype(np.int64))
+        assert n[h] == len(om)
+        np.testing.assert_array_equal(m[h, :n[h]], om)
+    assert (n[[1, 5, 6]] == -7).all()
+
+
+@pytest.mark.parametrize("wide,group", [(0, 2), (1, 0)])
+def test_chunks_that_cannot_be_joined(emu_exe, tmp_path, wide, group):
+    """Lists that outgrow a chunk's, or that together could outgrow the most a
+    list may hold, and a part of the buffer that is too small: the haplotype
+    gets the retry mark."""
+    from oracle import restate as R
+    rng = np.random.default_rng(15)
+    K, M = 2200, 96
+    sm = pack_rows((rng.random((M, K)) < 0.5).astype(np.uint8), W(K))
+    gt = rng.integers(0, 2, (2, M)).astype(np.uint8)
+    gt[0, 8:17] = 3
+    gt[0, 70:80] = 3
+    ph = pack_rows((rng.random((4, M)) < 0.5).astype(np.uint8), W(M))
+    compr, c0, _ = R.pbwt(sm, K)
+    want = [R.smmatches(compr, c0, M, K, ph[h], np.flatnonzero(gt[h // 2] == 3).astype(np.int64)) for h in range(4)]
+    for slots, again in ((8, []), (0, [0, 1])):
+        m, n, status, _ = run(emu_exe, tmp_path / f"k{slots}", compr, ph, gt, K, wide, 4, group, slots, chunks=2)
+        assert status == 0 and list(np.flatnonzero(n == -2)) == again
+        for h in set(range(4)) - set(again):
+            assert n[h] == len(want[h])
+            np.testing.assert_array_equal(m[h, :n[h]], want[h])
+    _, n, status, _ = run(emu_exe, tmp_path / "small", compr, ph, gt, K, wide, 4, group, 8, cap=6, chunks=3)
+    assert status == 0 and (n[2:] == -2).all()
+    gt[0, 8:21] = 3    # more than 4,096 entries in one piece
+    gt[0, 70:83] = 3
+    _, n, status, _ = run(emu_exe, tmp_path / "large", compr, ph, gt, K, wide, 4, group, 8, chunks=2)
+    one = run(emu_exe, tmp_path / "one", compr, ph, gt, K, wide, 4, group, 8)
+    assert ((one[1] == -2) <= (n == -2)).all() and status == one[2] == 0
 
 
 def test_haploid_golden(emu_exe, tmp_path):

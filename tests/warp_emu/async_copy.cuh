@@ -4,6 +4,7 @@
 #pragma once
 #include "emu.h"
 namespace eimp {
+constexpr int MBAR_POLLS = 1 << 28;   // polls are far shorter here than on the device
 struct EmuMbar { std::atomic<int> pending; std::atomic<short> phase; short count; };
 static_assert(sizeof(EmuMbar) == 8, "stored in a barrier's 64 bits");
 inline EmuMbar *emu_mbar(uint64_t *b) { return reinterpret_cast<EmuMbar *>(b); }
@@ -20,6 +21,10 @@ inline void mbar_arrive(uint64_t *b) {
     }
 }
 inline void mbar_expect(uint64_t *, unsigned) {}
+inline bool mbar_try(uint64_t *b, unsigned parity) {
+    sched_yield();
+    return (unsigned)(emu_mbar(b)->phase.load() & 1) != (parity & 1u);
+}
 inline bool mbar_wait(uint64_t *b, unsigned parity) {
     while ((unsigned)(emu_mbar(b)->phase.load() & 1) == (parity & 1u)) sched_yield();
     return true;

@@ -1,12 +1,13 @@
 // Runs smm_list_kernel (generated host copy of eimp_b200/csrc/smm_list.cu)
 // under the warp emulator, whole CTAs one after the other.
 //
-//   smm_list_emu <dir> <wide> <warps> <group> <pool slots>
+//   smm_list_emu <dir> <wide> <warps> <group> <pool slots> [chunks]
 //
 // <dir> holds params_i.bin (nhaps, M, K, cap, nrows, use_hapmap), compr.bin,
 // phased.bin, gt.bin and hapmap.bin as smm_main.cpp takes them; wide: 64-bit
 // intervals; warps: haplotypes per CTA; group: rows per ring stage (0: read
-// in place).  Outputs: o_matches.bin, o_nmatch.bin, o_status.bin (status,
+// in place); chunks: parts of a haplotype's sites, joined by
+// smm_list_join_kernel when there are several.  Outputs: o_matches.bin, o_nmatch.bin, o_status.bin (status,
 // pool slots taken).  Exit status 3: a divergent warp collective.
 #include "smm_list_emu.cpp"
 
@@ -40,7 +41,7 @@ template <class T> static void wr(const std::string &d, const char *name, const 
     fclose(f);
 }
 
-template <bool WIDE> static int go(const std::string &d, int warps, int group, int slots) {
+template <bool WIDE> static int go(const std::string &d, int warps, int group, int slots, int chunks) {
     using namespace eimp;
     const auto pi = rd<int32_t>(d, "params_i.bin");
     const int nhaps = pi[0], M = pi[1], K = pi[2], cap = pi[3], nrows = pi[4];
@@ -60,9 +61,9 @@ template <bool WIDE> static int go(const std::string &d, int warps, int group, i
     typedef SlList<WIDE, SL_POOL> Pool;
     std::vector<uint64_t> gpool(slots * sizeof(Pool) / 8, 0x5a5a5a5a5a5a5a5aull);
     const size_t rowbytes = (size_t)((K + 31) / 32) * 8, stage = group ? (group * rowbytes + 30) & ~(size_t)15 : 0;
-    const size_t smb = 2 * SL_STAGES * 8 + SL_STAGES * stage + (size_t)warps * sizeof(SlList<WIDE, SL_CAP>);
+    const size_t smb = SL_HEAD + SL_STAGES * stage + (size_t)warps * sizeof(SlList<WIDE, SL_CAP>);
     const int nthreads = 32 * (warps + (group ? 1 : 0));
-    for (int b = 0; b < (nhaps + warps - 1) / warps; b++) {
+    for (int b = 0; b < (nhaps + warps - 1) / warps; b++) for (int chunk = 0; chunk < chunks; chunk++) {
         uint8_t *smem = (uint8_t *)aligned_alloc(16, (smb + 15) / 16 * 16);
         memset(smem, 0x5A, smb);
         std::vector<EmuWarp> ws(nthreads / 32);
@@ -73,6 +74,7 @@ template <bool WIDE> static int go(const std::string &d, int warps, int group, i
             lanes.emplace_back([&, t] {
                 threadIdx.x = t;
                 blockIdx.x = b;
+                blockIdx.y = chunk;
                 blockDim.x = nthreads;
                 emu_warp = &ws[t / 32];
                 emu_block = &block;
@@ -80,10 +82,24 @@ template <bool WIDE> static int go(const std::string &d, int warps, int group, i
                 smm_list_kernel<WIDE>(compr, M, K, phased.data(), (int)eimp_W(M), gt.data(), nhaps,
                                       hapmap.empty() ? nullptr : hapmap.data(), matches.data(), cap, nmatch.data(),
                                       &status, warps, group, (unsigned)stage, slots ? (Pool *)gpool.data() : nullptr,
-                                      slots, &gnext);
+                                      slots, &gnext, chunks);
             });
         for (auto &x : lanes) x.join();
         free(smem);
+    }
+    for (int b = 0; chunks > 1 && b < nhaps; b++) {
+        EmuWarp w;
+        std::vector<std::thread> lanes;
+        for (int t = 0; t < 32; t++)
+            lanes.emplace_back([&, t] {
+                threadIdx.x = t;
+                blockIdx.x = b;
+                blockDim.x = 32;
+                emu_warp = &w;
+                smm_list_join_kernel(M, hapmap.empty() ? nullptr : hapmap.data(), matches.data(), cap, nmatch.data(),
+                                     &status, chunks);
+            });
+        for (auto &x : lanes) x.join();
     }
     free(compr);
     wr(d, "o_matches.bin", matches);
@@ -94,7 +110,8 @@ template <bool WIDE> static int go(const std::string &d, int warps, int group, i
 }
 
 int main(int argc, char **argv) {
-    if (argc < 6) { fprintf(stderr, "usage: %s <dir> <wide> <warps> <group> <slots>\n", argv[0]); return 1; }
+    if (argc < 6) { fprintf(stderr, "usage: %s <dir> <wide> <warps> <group> <slots> [chunks]\n", argv[0]); return 1; }
     const int warps = atoi(argv[3]), group = atoi(argv[4]), slots = atoi(argv[5]);
-    return atoi(argv[2]) ? go<true>(argv[1], warps, group, slots) : go<false>(argv[1], warps, group, slots);
+    const int chunks = argc > 6 ? atoi(argv[6]) : 1;
+    return atoi(argv[2]) ? go<true>(argv[1], warps, group, slots, chunks) : go<false>(argv[1], warps, group, slots, chunks);
 }
