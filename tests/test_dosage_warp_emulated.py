@@ -162,6 +162,38 @@ def test_dosages_shortcut_and_wide_tiles(emu_exe, tmp_path):
     assert taken == {False, True}
 
 
+@pytest.mark.parametrize("copies", [5, 6, 7, 31, 32, 33, 64, 65, 96, 97, 128, 129])
+def test_dosages_slot_counts(emu_exe, tmp_path, copies):
+    """Targets that copy a haplotype of which the panel holds this many, plus
+    ones that change to another group half way: covering matches with slots
+    around every chunk's edge, some of a match's in two chunks."""
+    from oracle import restate as R
+    rng = np.random.default_rng(copies)
+    Mref, nh = 400, copies + 40
+    typed = np.sort(rng.choice(Mref, 60, replace=False)).astype(np.int64)
+    base = (rng.random((2, Mref)) < 0.5).astype(np.uint8)
+    ref = (rng.random((nh, Mref)) < 0.5).astype(np.uint8)
+    ref[:copies] = base[0]
+    ref[copies:copies + 20] = base[1]
+    untyped = np.setdiff1d(np.arange(Mref), typed)
+    flip = rng.random((nh, len(untyped))) < 0.1
+    ref[:, untyped] ^= flip.astype(np.uint8)
+    af = ref.mean(axis=0).astype(np.float32)
+    sm_full = pack_rows(ref.T.copy(), W(nh))
+    sm_typed = np.ascontiguousarray(sm_full[typed])
+    mixed = np.where(np.arange(Mref) < Mref // 2, base[0], base[1])
+    th = np.stack([base[0], mixed])[:, typed]
+    gt = (th[0::2] + th[1::2]).astype(np.uint8)
+    phased = pack_rows(th, W(len(typed)))
+    compr, c0, ap = R.pbwt(sm_typed, nh, absperm=True)
+    matches = [R.smmatches(compr, c0, len(typed), nh, phased[h], np.zeros(0, np.int64)) for h in range(2)]
+    assert max(int((m[:, 3] - m[:, 2]).max()) + 1 for m in matches) >= copies
+    od, ob = oracle_full(matches, ap, sm_full, typed, af, nh, phased, gt)
+    dos, bits = run_kernel(emu_exe, tmp_path / "s", matches, ap, sm_full, typed, af, phased, gt, 0, Mref)
+    np.testing.assert_array_equal(dos, od)
+    np.testing.assert_array_equal(unpack_rows(bits, Mref), unpack_rows(ob, Mref))
+
+
 def test_dosages_long_match_lists(emu_exe, tmp_path):
     """Targets unrelated to a random panel: short set-maximal matches, hundreds
     per haplotype, so every span's window start is found by the search over
