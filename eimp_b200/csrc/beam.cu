@@ -553,45 +553,36 @@ __device__ __forceinline__ void beam_walk(const Ctx &c, WS &w) {
     }
 }
 
+// (short code on purpose: a job in flight at a time and no unrolled copies; with
+// two jobs side by side, four times the code, 1,000 targets of 5,000 sites took
+// 64 instead of 59 ms a pass, three CTAs per SM fetching their instructions)
 // the paths that split: this warp's share of the copies of rings (with the
 // copy's own entry pushed) and extension-1 intervals
 __device__ __forceinline__ void beam_copy(const Ctx &c, const WS &w, int first, int stride) {
     const int lane = lane_id(), phs = w.phsize;
 #pragma unroll 1
-    for (int k = first; k < w.njob; k += 2 * stride) {   // two at a time, their loads in flight together
-        float4 x[2];
-        uint32_t v[2][4];
+    for (int k = first; k < w.njob; k += stride) {
+        const Job &j = w.job[k];
+        const float *a = c.ph(j.src);
+        const uint32_t *s = c.iv(j.src, j.buf);
+        float *b = c.ph(j.dst);
+        uint32_t *d = c.iv(j.dst, 0);
+        const int start = j.start, n = j.n;
+        const float p = j.p;
+#pragma unroll 1
+        for (int i = lane; i < max(phs, n); i += 64) {   // two words of each per lane in flight
+            float x[2];
+            uint32_t v[2];
 #pragma unroll
-        for (int u = 0; u < 2; u++) {
-            if (k + u * stride >= w.njob) continue;
-            const Job &j = w.job[k + u * stride];
-            const float *a = c.ph(j.src);
-            const uint32_t *s = c.iv(j.src, j.buf);
-            if (phs >= 4) {
-                if (lane < phs / 4) x[u] = reinterpret_cast<const float4 *>(a)[lane];
-            } else if (lane < phs) x[u].x = a[lane];
+            for (int u = 0; u < 2; u++) {
+                if (i + 32 * u < phs) x[u] = a[i + 32 * u];
+                if (i + 32 * u < n) v[u] = s[i + 32 * u];
+            }
 #pragma unroll
-            for (int q = 0; q < 4; q++)
-                if (lane + 32 * q < j.n) v[u][q] = s[lane + 32 * q];
-        }
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-            if (k + u * stride >= w.njob) continue;
-            const Job &j = w.job[k + u * stride];
-            float *b = c.ph(j.dst);
-            uint32_t *d = c.iv(j.dst, 0);
-            if (phs >= 4) {
-                if (lane < phs / 4) {
-                    if (j.start >> 2 == lane) {
-                        const int r = j.start & 3;
-                        if (r == 0) x[u].x = j.p; else if (r == 1) x[u].y = j.p; else if (r == 2) x[u].z = j.p; else x[u].w = j.p;
-                    }
-                    reinterpret_cast<float4 *>(b)[lane] = x[u];
-                }
-            } else if (lane < phs) b[lane] = lane == j.start ? j.p : x[u].x;
-#pragma unroll
-            for (int q = 0; q < 4; q++)
-                if (lane + 32 * q < j.n) d[lane + 32 * q] = v[u][q];
+            for (int u = 0; u < 2; u++) {
+                if (i + 32 * u < phs) b[i + 32 * u] = i + 32 * u == start ? p : x[u];
+                if (i + 32 * u < n) d[i + 32 * u] = v[u];
+            }
         }
     }
 }
@@ -1950,7 +1941,12 @@ __global__ void __launch_bounds__(BEAM_SM_CTAS * 32 * BEAM_WARPS, 1) beam_kernel
 
 // The launch: with a target or less per SM, one CTA of BEAM_MAX_WARPS warps on
 // each; with more, CTAs of BEAM_WARPS warps, as many per SM as the targets fill, at
-// most BEAM_SM_CTAS.  The shared memory that is left becomes haplotype-path slots.
+// most BEAM_SM_CTAS.  The shared memory that is left becomes haplotype-path slots:
+// all of it with a target or less per SM, a BEAM_SM_CTAS-th with more -- a second
+// context's beams then find room beside the last targets of the first (192
+// targets of 32,000 sites, three contexts in turn: 57.5 -> 45.5 ms a pass), and
+// slots that go to the arena for it cost little (1,000 targets of 5,000 sites,
+// one CTA per SM: 107 ms with all slots in shared memory, 112 with 12).
 struct BeamShape { int warps, ctas; size_t smem; };
 
 static size_t beam_smem(const BeamParams &p, const ArenaLayout &al, int warps) {
@@ -1974,7 +1970,8 @@ static bool beam_shape(const BeamParams &p, ArenaLayout &al, int ntgt, BeamShape
     if (base > (size_t)lim) return false;
     size_t room;   // of each CTA, 1 KB of it the system's
     for (;; per--) {
-        room = (size_t)sm / per - 1024;
+        room = (size_t)sm / (per > 1 ? BEAM_SM_CTAS : 1) - 1024;
+        if (room < base) room = (size_t)sm / per - 1024;
         if (room > (size_t)lim) room = (size_t)lim;
         if (per == 1 || base <= room) break;
     }
