@@ -273,6 +273,13 @@ __global__ void __launch_bounds__(256) monos_calls_kernel(
     const int32_t *__restrict__ besthaps, int K, const float *__restrict__ cm, float cMmaxsplit,
     uint64_t *__restrict__ monos, int32_t *__restrict__ splits, int32_t *__restrict__ calls,
     float *__restrict__ cmdiffs, int32_t *__restrict__ nsplits, int32_t *__restrict__ ncalls,
+    const uint8_t *__restrict__ tgt_haploid);
+
+__device__ __forceinline__ void monos_calls(
+    const uint8_t *__restrict__ gt, int M, const uint64_t *__restrict__ hapmajor, int wM,
+    const int32_t *__restrict__ besthaps, int K, const float *__restrict__ cm, float cMmaxsplit,
+    uint64_t *__restrict__ monos, int32_t *__restrict__ splits, int32_t *__restrict__ calls,
+    float *__restrict__ cmdiffs, int32_t *__restrict__ nsplits, int32_t *__restrict__ ncalls,
     const uint8_t *__restrict__ tgt_haploid) {
     extern __shared__ unsigned long long smo[];
     unsigned long long *sand = smo, *sor = smo + wM;
@@ -292,7 +299,15 @@ __global__ void __launch_bounds__(256) monos_calls_kernel(
         int sl = slices == 1 ? 0 : idx / wM;
         if (w < wM && sl < slices) {
             unsigned long long a = ~0ull, o = 0ull;
-            for (int k = sl; k < K; k += slices) {
+            int k = sl;
+            for (; k + 7 * slices < K; k += 8 * slices) {   // eight haplotypes' words in flight
+                unsigned long long x[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) x[u] = hapmajor[(size_t)bh[k + u * slices] * wM + w];
+#pragma unroll
+                for (int u = 0; u < 8; u++) { a &= x[u]; o |= x[u]; }
+            }
+            for (; k < K; k += slices) {
                 unsigned long long x = hapmajor[(size_t)bh[k] * wM + w];
                 a &= x; o |= x;
             }
@@ -332,11 +347,23 @@ __global__ void __launch_bounds__(256) monos_calls_kernel(
         const unsigned f = __ballot_sync(FULL, b + lane < M && g[b + lane] == 1);
         if (f) { m0 = b + __ffs((int)f) - 1; break; }
     }
+    // two chunks ahead, or their latency is that of the whole loop
+    uint8_t gq[2];
+    float cq[2];
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        const int m = m0 + 32 * u + lane;
+        gq[u] = m < M ? g[m] : 3;
+        cq[u] = m < M ? cm[m] : 0.0f;
+    }
     for (int b = m0; b < M; b += 32) {
         const int m = b + lane;
-        const uint8_t c = m < M ? g[m] : 3;
+        const uint8_t c = gq[0];
         const bool mono = m < M && ((sand[m >> 6] >> (m & 63)) & 1ull);
-        const float cmv = m < M ? cm[m] : 0.0f;
+        const float cmv = cq[0];
+        gq[0] = gq[1]; cq[0] = cq[1];
+        gq[1] = m + 64 < M ? g[m + 64] : 3;
+        cq[1] = m + 64 < M ? cm[m + 64] : 0.0f;
         const bool het = !mono && c == 1, hom = !mono && c != 1 && c != 3;
         const unsigned hets = __ballot_sync(FULL, het);
         unsigned spl = hets;   // the chunk's splits known so far
@@ -374,16 +401,42 @@ __global__ void __launch_bounds__(256) monos_calls_kernel(
     if (lane == 0) { nsplits[t] = S; ncalls[t] = C; }
 }
 
+// What bounds it: the latency of the K haplotypes' rows and of one warp's walk
+// over the sites, so rows are read eight at a time and sites two chunks ahead.
+// With one CTA to an SM or two, four times the threads read rows: 192 targets of
+// 32,000 sites, K = 4,096 2.34 -> 0.86 ms, 96 of 10,000, K = 8,192 2.31 -> 0.42
+// ms, one of 2,000, K = 1,024 0.12 -> 0.055 ms; 1,000 of 5,000 sites
+// 0.37 ms with 256 threads, 0.60 with 1,024.
+__global__ void __launch_bounds__(256) monos_calls_kernel(
+    const uint8_t *__restrict__ gt, int M, const uint64_t *__restrict__ hapmajor, int wM,
+    const int32_t *__restrict__ besthaps, int K, const float *__restrict__ cm, float cMmaxsplit,
+    uint64_t *__restrict__ monos, int32_t *__restrict__ splits, int32_t *__restrict__ calls,
+    float *__restrict__ cmdiffs, int32_t *__restrict__ nsplits, int32_t *__restrict__ ncalls,
+    const uint8_t *__restrict__ tgt_haploid) {
+    monos_calls(gt, M, hapmajor, wM, besthaps, K, cm, cMmaxsplit, monos, splits, calls, cmdiffs, nsplits, ncalls, tgt_haploid);
+}
+__global__ void __launch_bounds__(1024) monos_calls_wide_kernel(
+    const uint8_t *__restrict__ gt, int M, const uint64_t *__restrict__ hapmajor, int wM,
+    const int32_t *__restrict__ besthaps, int K, const float *__restrict__ cm, float cMmaxsplit,
+    uint64_t *__restrict__ monos, int32_t *__restrict__ splits, int32_t *__restrict__ calls,
+    float *__restrict__ cmdiffs, int32_t *__restrict__ nsplits, int32_t *__restrict__ ncalls,
+    const uint8_t *__restrict__ tgt_haploid) {
+    monos_calls(gt, M, hapmajor, wM, besthaps, K, cm, cMmaxsplit, monos, splits, calls, cmdiffs, nsplits, ncalls, tgt_haploid);
+}
+
 cudaError_t launch_monos_calls(const uint8_t *gt, int ntgt, int M, const uint64_t *hapmajor, int wM,
                                const int32_t *besthaps, int K, const float *cm, float cMmaxsplit, uint64_t *monos,
                                int32_t *splits, int32_t *calls, float *cmdiffs, int32_t *nsplits, int32_t *ncalls,
                                const uint8_t *tgt_haploid, cudaStream_t st) {
     size_t sm = (size_t)2 * wM * sizeof(uint64_t);
-    if (sm > 48 * 1024) {
-        cudaError_t e = ensure_dynamic_smem((const void *)monos_calls_kernel, sm);
-        if (e != cudaSuccess) return e;
-    }
-    monos_calls_kernel<<<ntgt, 256, sm, st>>>(gt, M, hapmajor, wM, besthaps, K, cm, cMmaxsplit, monos, splits, calls,
+    int dev = 0, nsm = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    const bool many = ntgt > 2 * nsm;
+    const auto kern = many ? monos_calls_kernel : monos_calls_wide_kernel;
+    if (sm > 48 * 1024 && (e = ensure_dynamic_smem((const void *)kern, sm)) != cudaSuccess) return e;
+    kern<<<ntgt, many ? 256 : 1024, sm, st>>>(gt, M, hapmajor, wM, besthaps, K, cm, cMmaxsplit, monos, splits, calls,
                                               cmdiffs, nsplits, ncalls, tgt_haploid);
     return cudaGetLastError();
 }
@@ -599,6 +652,14 @@ cudaError_t launch_cref(const uint8_t *gt, int ntgt, int M, const uint64_t *hapm
 // the gather to the placement.  The next row is copied into shared memory asynchronously
 // while the current one is processed.  The forward CTA also writes each
 // row's zero count.
+//
+// What bounds it: with many CTAs on an SM the instructions and the bank
+// conflicts of the gathers and placements, with few the chain of rows.  Where
+// the launch has few warps a word is shared by SUB threads, each with a run of
+// its positions (WPT = 1): one target of 2,000 sites, K = 1,024, SUB 1 -> 4
+// 0.39 -> 0.25 ms, 100 of them 0.39 -> 0.28 ms.  With ten warps per SM before
+// the split two threads to a word are already slower: 192 targets of 32,000
+// sites, K = 4,096, 9.9 -> 10.9 ms, 96 of 10,000, K = 8,192, 3.7 -> 4.5 ms.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -614,16 +675,17 @@ __device__ __forceinline__ int pswz(int p) { return p ^ ((p >> 5) & 31); }
 // 31, the block's swizzle): positions 2i and 2i+1 sit in the 32-bit pair
 // i ^ (key >> 1) of the block, swapped when key is odd, so sixteen 32-bit
 // loads (the 32 lanes of a warp on 32 different banks) fetch the block.  The
-// pairs go to hp in position order; the bits are pushed from position 31
-// down to 0.
-__device__ __forceinline__ uint32_t pbwt_gather(const uint32_t *__restrict__ pw, int key,
-                                                const uint32_t *__restrict__ row, uint32_t hp[16]) {
+// pairs go to hp in position order; the bits are pushed from the last position
+// down.  PAIRS of them from pair i0 on: a thread's share of the word.
+template <int PAIRS>
+__device__ __forceinline__ uint32_t pbwt_gather(const uint32_t *__restrict__ pw, int key, int i0,
+                                                const uint32_t *__restrict__ row, uint32_t hp[PAIRS]) {
     const int k2 = key >> 1;
     const unsigned rot = (unsigned)(key & 1) << 4;
     uint32_t b = 0u;
 #pragma unroll
-    for (int i = 15; i >= 0; i--) {
-        const uint32_t v = pw[i ^ k2];
+    for (int i = PAIRS - 1; i >= 0; i--) {
+        const uint32_t v = pw[(i0 + i) ^ k2];
         const uint32_t x = __funnelshift_r(v, v, rot);
         hp[i] = x;
         const uint32_t h0 = x & 0xffffu, h1 = x >> 16;
@@ -634,14 +696,14 @@ __device__ __forceinline__ uint32_t pbwt_gather(const uint32_t *__restrict__ pw,
     return b;
 }
 
-// Places the haplotypes of one block (hp, data word b) in the next prefix
+// Places N haplotypes of one block (hp, their bits b) in the next prefix
 // order: a zero at the next zero place dz, a one at the next one place d1
 // (stable).  CHECK: only the first nv positions exist (the block holding K).
-template <bool CHECK>
-__device__ __forceinline__ void pbwt_place(uint16_t *__restrict__ nperm, const uint32_t hp[16], uint32_t b, int nv,
+template <bool CHECK, int N>
+__device__ __forceinline__ void pbwt_place(uint16_t *__restrict__ nperm, const uint32_t hp[N / 2], uint32_t b, int nv,
                                            int &dz, int &d1) {
 #pragma unroll
-    for (int j = 0; j < 32; j++) {
+    for (int j = 0; j < N; j++) {
         if (!CHECK || j < nv) {
             const uint32_t x = hp[j >> 1];
             const uint16_t h = (uint16_t)((j & 1) ? x >> 16 : x & 0xffffu);
@@ -653,7 +715,7 @@ __device__ __forceinline__ void pbwt_place(uint16_t *__restrict__ nperm, const u
     }
 }
 
-template <int WPT>
+template <int WPT, int SUB = 1>
 __global__ void __launch_bounds__(1024) pbwt_kernel(const uint64_t *__restrict__ cref,
                                                     const int64_t *__restrict__ rowoff, int K,
                                                     uint32_t *__restrict__ pbwt, size_t rowstride, int emit_padded,
@@ -673,7 +735,10 @@ __global__ void __launch_bounds__(1024) pbwt_kernel(const uint64_t *__restrict__
     const int Mp = (int)(rowoff[t + 1] - r0);
     const uint64_t *rows = cref + (size_t)r0 * wK;
     uint32_t *out = pbwt + (size_t)(2 * r0 + (dir ? Mp : 0)) * rowstride;
-    const int w0 = tid * WPT;                      // the thread's first word
+    constexpr int N = 32 / SUB;                    // positions of a thread in a word
+    static_assert(SUB == 1 || WPT == 1, "a thread has several words or a part of one");
+    const int w0 = tid / SUB * WPT;                // the thread's first word
+    const int p0 = tid % SUB * N;                  // its first position in it
     const int nchunk = wK / 2;                     // 16-byte pieces of a row
     // identity order; the padding positions past K hold haplotype 0 in both
     // arrays (never written later, never used for a bit)
@@ -698,19 +763,25 @@ __global__ void __launch_bounds__(1024) pbwt_kernel(const uint64_t *__restrict__
         // haplotypes of their positions (two per register, in position order)
         // kept for the placement
         uint32_t word[WPT];
-        uint32_t hp[WPT][16];
+        uint32_t hp[WPT][N / 2];
         int zsum = 0;
 #pragma unroll
         for (int q = 0; q < WPT; q++) {
             const int w = w0 + q;
             uint32_t b = ~0u;
             if (w < nwords) {
-                b = pbwt_gather(reinterpret_cast<const uint32_t *>(perm + w * 32), w & 31, row, hp[q]);
-                const int past = K - w * 32;   // positions past K read as 1 (the row format's padding)
-                if (past < 32) b |= ~0u << past;
+                b = pbwt_gather<N / 2>(reinterpret_cast<const uint32_t *>(perm + w * 32), w & 31, p0 / 2, row, hp[q]);
+                const int past = K - w * 32 - p0;   // positions past K read as 1 (the row format's padding)
+                if (past < N) b |= past > 0 ? ~0u << past : ~0u;
+                if (SUB > 1) b |= ~0u << (N & 31);
                 zsum += __popc(~b);
             }
             word[q] = b;
+        }
+        uint32_t whole = 0u;   // the word of SUB threads together
+        if (SUB > 1) {
+            whole = (word[0] & ~(~0u << (N & 31))) << p0;
+            for (int o = 1; o < SUB; o <<= 1) whole |= __shfl_xor_sync(0xffffffffu, whole, o);
         }
         // zeros before the thread's words: warp scan, then the warps' totals
         int inc = zsum;
@@ -730,10 +801,10 @@ __global__ void __launch_bounds__(1024) pbwt_kernel(const uint64_t *__restrict__
             const uint32_t b = word[q];
             // the next zero's place (zeros so far) and the next one's (cnt0 +
             // ones so far)
-            int dz = zb, d1 = cnt0 + w * 32 - zb;
-            if (w * 32 + 32 <= K) pbwt_place<false>(nperm, hp[q], b, 32, dz, d1);
-            else pbwt_place<true>(nperm, hp[q], b, K - w * 32, dz, d1);
-            reinterpret_cast<uint2 *>(o)[w] = make_uint2(b, (uint32_t)dz);
+            int dz = zb, d1 = cnt0 + w * 32 + p0 - zb;
+            if (w * 32 + p0 + N <= K) pbwt_place<false, N>(nperm, hp[q], b, N, dz, d1);
+            else pbwt_place<true, N>(nperm, hp[q], b, K - w * 32 - p0, dz, d1);
+            if (SUB == 1 || p0 + N == 32) reinterpret_cast<uint2 *>(o)[w] = make_uint2(SUB == 1 ? b : whole, (uint32_t)dz);
             zb = dz;
         }
         if (emit_padded)
@@ -751,15 +822,16 @@ static size_t pbwt_smem(int K) {
 }
 
 template <int WPT>
-static cudaError_t launch_pbwt_w(const uint64_t *cref, int32_t *count0, const int64_t *rowoff, int ntgt, int K,
-                                 uint32_t *pbwt, size_t rowstride, int emit_padded, const int *skip,
+static cudaError_t launch_pbwt_w(int sub, const uint64_t *cref, int32_t *count0, const int64_t *rowoff, int ntgt,
+                                 int K, uint32_t *pbwt, size_t rowstride, int emit_padded, const int *skip,
                                  cudaStream_t st) {
     const int nwords = (K + 31) / 32;
-    const int nthreads = ((nwords + WPT - 1) / WPT + 31) / 32 * 32;
+    const int nthreads = ((nwords + WPT - 1) / WPT * sub + 31) / 32 * 32;
     const size_t sm = pbwt_smem(K);
-    cudaError_t e = ensure_dynamic_smem((const void *)pbwt_kernel<WPT>, sm);
+    const auto kern = sub == 4 ? pbwt_kernel<1, 4> : sub == 2 ? pbwt_kernel<1, 2> : pbwt_kernel<WPT>;
+    cudaError_t e = ensure_dynamic_smem((const void *)kern, sm);
     if (e != cudaSuccess) return e;
-    pbwt_kernel<WPT><<<2 * ntgt, nthreads, sm, st>>>(cref, rowoff, K, pbwt, rowstride, emit_padded, count0, skip);
+    kern<<<2 * ntgt, nthreads, sm, st>>>(cref, rowoff, K, pbwt, rowstride, emit_padded, count0, skip);
     return cudaGetLastError();
 }
 
@@ -768,8 +840,15 @@ cudaError_t launch_pbwt(const uint64_t *cref, int32_t *count0, const int64_t *ro
     // the 8-byte pair stores need 8-byte aligned rows
     if (K < 1 || K > 65536 || rowstride % 2) return cudaErrorInvalidValue;
     const int nwords = (K + 31) / 32;
-    if (nwords <= 1024) return launch_pbwt_w<1>(cref, count0, rowoff, ntgt, K, pbwt, rowstride, emit_padded, skip, st);
-    return launch_pbwt_w<2>(cref, count0, rowoff, ntgt, K, pbwt, rowstride, emit_padded, skip, st);
+    int dev = 0, nsm = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    // threads to a word: several as long as they make no more than 8 warps per SM
+    const size_t warps = (size_t)2 * ntgt * ((nwords + 31) / 32), most = (size_t)8 * nsm;
+    const int sub = 4 * nwords <= 1024 && 4 * warps <= most ? 4 : 2 * nwords <= 1024 && 2 * warps <= most ? 2 : 1;
+    if (nwords <= 1024) return launch_pbwt_w<1>(sub, cref, count0, rowoff, ntgt, K, pbwt, rowstride, emit_padded, skip, st);
+    return launch_pbwt_w<2>(1, cref, count0, rowoff, ntgt, K, pbwt, rowstride, emit_padded, skip, st);
 }
 
 // ---------------------------------------------------------------------------

@@ -51,6 +51,28 @@ def emu_exe(tmp_path_factory):
     return str(exe)
 
 
+@pytest.fixture(scope="module", params=[2, 4])
+def emu_sub_exe(emu_exe, tmp_path_factory, request):
+    """The driver with several threads to a word."""
+    d = tmp_path_factory.mktemp("pbwt_sub_emu")
+    main = open(os.path.join(EMU, "pbwt_main.cpp")).read()
+    for a, b in [("pbwt_kernel<1>(", f"pbwt_kernel<1, {request.param}>("),
+                 ("nthreads = ((nwords + wpt - 1) / wpt + 31)", f"nthreads = (nwords * {request.param} + 31)")]:
+        assert main.count(a) == 1
+        main = main.replace(a, b)
+    (d / "main.cpp").write_text(main)
+    r = subprocess.run(["g++", "-std=c++20", "-O1", "-g", "-fsanitize=address,undefined",
+                        "-fno-sanitize-recover=undefined", "-I", EMU, "-I", os.path.dirname(emu_exe),
+                        str(d / "main.cpp"), "-o", str(d / "pbwt_sub_emu"), "-lpthread"], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-4000:]
+    return str(d / "pbwt_sub_emu")
+
+
+@pytest.mark.parametrize("K,nrows", [(4096, [9, 0, 5]), (1000, [7, 3]), (20, [6]), (33, [4]), (264, [5]), (64, [1, 2])])
+def test_pbwt_shared_words(emu_sub_exe, tmp_path, K, nrows):
+    test_pbwt_emulated(emu_sub_exe, tmp_path, K, 1, nrows)
+
+
 def _rows(rng, n, K):
     wK = W(K)
     dens = rng.choice([0.0, 0.02, 0.3, 0.5, 1.0], size=n, p=[0.1, 0.3, 0.25, 0.25, 0.1])
