@@ -9,8 +9,9 @@ at their current values), keeps the fastest and leaves it set on the group's
 context.  Knobs (eimp_set_launch_shape, include/eimp_gpu.h):
 
   dosage_span     64-site tiles per warp of the dosage kernel       4, 8, 16
-  smm_warps       target haplotypes per CTA of the match search     1, 2, 4
-  beam_slots_pct  warps of the persistent beam, % of the resident   100, 75, 50
+  smm_warps       target haplotypes per CTA of the match search
+                  (with set-maximal errors)                         1, 2, 4
+  beam_slots_pct  CTAs of the persistent beam, % of the resident    100, 75, 50
   smm_tree_pools  large match trees go on in global pools (1) or    1, 0
                   are redone by the retry launch (0)
 

@@ -1,4 +1,4 @@
-// Eagle2-style beam phasing over the condensed PBWT, one warp per target.
+// Eagle2-style beam phasing over the condensed PBWT, one CTA per target.
 //
 // Device restatement of Target::phaseExtPBWT (Target.cpp:291-777) with Beam
 // (Beam.cpp:41-837), BeamPath (BeamPath.cpp:29-291), HaplotypePath
@@ -51,11 +51,10 @@
 // of their own): it has to stay in the instruction cache.
 //
 // Measured on a B200 against one warp per target with everything but the beam
-// in the arena and five copies of the step's code (kernel times): one target
-// of 2,000 sites, K = 1,024 8.0 -> 2.1 ms; 100 of them 11.7 -> 3.6 ms; 192
-// targets of 32,000 sites, K = 4,096 148 -> 47 ms; 96 of 10,000 sites, K =
-// 8,192 83 -> 31 ms; 1,000 of 5,000 sites, whose beams outgrow shared memory,
-// 64 -> 59 ms.
+// in the arena and five copies of the step's code (kernel times): one target of
+// 2,000 sites, K = 1,024 8.0 -> 2.1 ms; 100 of them 11.7 -> 3.5 ms; 192 targets
+// of 32,000 sites, K = 4,096 148 -> 48 ms; 96 of 10,000 sites, K = 8,192 83 ->
+// 27 ms; 1,000 of 5,000 sites, whose beams outgrow shared memory, 64 -> 55 ms.
 #include <climits>
 
 #include "async_copy.cuh"

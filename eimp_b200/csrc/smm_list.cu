@@ -43,11 +43,11 @@
 // roots and goes on until its list is empty, so that together the chunks map
 // no entry twice.
 //
-// Measured on a B200, the general kernel (smm_compact_kernel), one site at a
-// time in one chunk, and now: 1,000 haplotypes x 5,000 sites of a
-// 10,000-haplotype panel 19.2, 4.6, 1.91 ms; 400 x 2,000 of 5,000 haplotypes
-// (now 0.32, one site at a time 1.34 ms); 128 x 3,000 of 20,000 haplotypes 11.7, 2.7, 0.39 ms; 64 x 2,000
-// of 200,000 haplotypes (rows in place) 12.9, 4.6, 0.40 ms.
+// Measured on a B200: the general kernel (smm_compact_kernel), one site at a
+// time in one chunk, and now.  1,000 haplotypes x 5,000 sites of a
+// 10,000-haplotype panel 19.2, 4.6, 1.91 ms; 128 x 3,000 of 20,000 haplotypes
+// 11.7, 2.7, 0.39 ms; 64 x 2,000 of 200,000 haplotypes (rows in place) 12.9, 4.6,
+// 0.40 ms; 400 x 2,000 of 5,000 haplotypes, the last two, 1.34, 0.32 ms.
 #include <climits>
 
 #include "async_copy.cuh"

@@ -214,8 +214,9 @@ int eimp_phase_haploid_targets(eimp_ctx *ctx, size_t ntgt, const uint8_t *haploi
 /* Launch shapes (no counterpart in the reference; the results do not depend
  * on them), per context, for the autotuner (eimp_b200/autotune.py):
  *   EIMP_SHAPE_DOSAGE_SPAN     64-site tiles per warp of the dosage kernel: 4, 8 [default] or 16
- *   EIMP_SHAPE_SMM_WARPS       warps (target haplotypes) per CTA of the match search: 1, 2 [default] or 4
- *   EIMP_SHAPE_BEAM_SLOTS_PCT  warps of the persistent beam launch, in % of the warps that can be
+ *   EIMP_SHAPE_SMM_WARPS       warps (target haplotypes) per CTA of the match search with set-maximal
+ *                              errors: 1, 2 [default] or 4 (without errors the launch decides)
+ *   EIMP_SHAPE_BEAM_SLOTS_PCT  CTAs (one target each) of the persistent beam launch, in % of those that can be
  *                              resident at once: 1..100 [default 100]
  *   EIMP_SHAPE_SMM_TREE_POOLS  1 [default]: a match tree that could outgrow its shared-memory pool
  *                              moves to a global-memory pool and its warp goes on; 0: such a
