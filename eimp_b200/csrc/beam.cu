@@ -1806,7 +1806,6 @@ __device__ __forceinline__ void beam_run(
             }
         }
         __syncwarp();
-        beam_command(c, w, ncmd, CMD_MEET);   // nothing of the pass before is in flight
         beam_init(c, w, p.doPrePhasing ? (pass == 2 ? rcons : cons) : nullptr, pass == 2, pass ? p.H : p.Hf, pass ? p.P : p.Pf, pass ? p.Delta : p.Deltaf);
         beam_command(c, w, ncmd, CMD_NEXT);
         int nci = 1, si = 1, rci = C - 2;   // the next call of pass 0 and 1, split site of pass 0, call of pass 2
@@ -1903,6 +1902,10 @@ __device__ __forceinline__ void beam_run(
                 rci--;
             }
         }
+        // the other warps are done with the pass: the copies of the paths that
+        // split last write the interval pool, the heaps' storage, and the next
+        // pass starts with new paths in it
+        beam_command(c, w, ncmd, CMD_MEET);
         if (pass == 0 && !err && lane == 0)
             constraint_heaps(reinterpret_cast<Hel *>(c.ivg), cons, phaseProbs, c.calls, S, p.minfixsize, p.maxfixsize,
                              p.minfixthr, p.maxfixthr);
