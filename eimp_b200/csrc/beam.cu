@@ -78,6 +78,7 @@ constexpr int HTS = 1 << HTS_BITS;   // merge hash table entries (load <= 1/2)
 static_assert(BPMAX < HTS, "the merge table must never fill");
 constexpr int WITEMS = 256;  // (path, step) items of a walk whose terms a warp holds at once
 constexpr int FWORDS = (4 * PMAX + 8 + 31) / 32;   // words of the free-slot mask
+static_assert(FWORDS <= 32, "a lane stores a word of it");
 
 struct HPh {   // HaplotypePath
     unsigned long long d0, d1;   // BooleanHistory data (fill mask applied)
@@ -741,7 +742,6 @@ __device__ __forceinline__ void beam_apply_hap(const Ctx &c, WS &w) {
 #pragma unroll 1
         while (k < ncp) {
             if (!f) {
-                if (lane == 0) w.fm[wi] = 0u;
                 if (++wi == FWORDS) break;
                 f = w.fm[wi];
                 continue;
@@ -750,7 +750,9 @@ __device__ __forceinline__ void beam_apply_hap(const Ctx &c, WS &w) {
             f &= f - 1;
             k++;
         }
-        if (wi < FWORDS && lane == 0) w.fm[wi] = f;
+        __syncwarp();   // the mask changes when all lanes have read it
+        if (lane < wi) w.fm[lane] = 0u;
+        if (lane == wi && wi < FWORDS) w.fm[wi] = f;
         if (k < ncp) {
             if (lane == 0) w.err |= EIMP_ERR_BEAM_CAPACITY;
             __syncwarp();

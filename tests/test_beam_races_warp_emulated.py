@@ -90,3 +90,10 @@ def test_heaps_after_the_last_copies(emu_exe, tmp_path):
     """The constraint heaps are filled only when no path is being copied."""
     got = reports(emu_exe, tmp_path, 16, True, range(20, 30))
     assert not [s for s in got if any(f.startswith(("heap_", "constraint_heaps", "hswap")) for f in s)], got
+
+
+@pytest.mark.parametrize("prephase,cuts", [(False, range(40, 43)), (True, range(24, 26))])
+def test_free_slots_read_before_they_change(emu_exe, tmp_path, prephase, cuts):
+    """The free-slot mask: every lane has read it before a lane stores it."""
+    got = reports(emu_exe, tmp_path, 16, prephase, cuts)
+    assert not [s for s in got if "beam_apply_hap" in s], got
