@@ -338,9 +338,11 @@ __device__ __forceinline__ int hp_required(const HPh &h, const Cons &cn) {
 // path whose probability has left 2^-20 .. 2^20
 __device__ __noinline__ void scale_ring(float *ph, int start, int niv, int pm, int e) {
     const double f = pow2i(-e);
-    for (int i = lane_id(); i <= niv; i += 32) {
+    // a full path of a history as long as the ring: entry niv is entry 0 again
+    for (int i = lane_id(); i <= min(niv, pm); i += 32) {
         float *x = &ph[(i + start) & pm];
-        *x = (float)((double)*x * f);
+        const float y = (float)((double)*x * f);
+        *x = i + pm < niv ? (float)((double)y * f) : y;
     }
     __syncwarp();
 }

@@ -51,7 +51,7 @@ def emu_exe(tmp_path_factory):
     return str(exe)
 
 
-def reports(exe, d, P, prephase, cuts):
+def reports(exe, d, P, prephase, cuts, H=8):
     """The sanitizer's reports, as lists of the functions on their stacks, for
     the panel's first target cut after each of the given numbers of split
     sites."""
@@ -72,7 +72,8 @@ def reports(exe, d, P, prephase, cuts):
                  count0=np.zeros(sum(map(len, crefs)), np.int32), rows=np.array([len(c) for c in crefs]), K=K, P=P,
                  prephase=prephase)
     pi = np.fromfile(os.path.join(d, "params_i.bin"), np.int32)
-    pi[3], pi[5], pi[6], pi[8] = 8, 4, 8, 0   # histories of 8: the heaps reach over several paths' buffers
+    # short histories: the heaps reach over several paths' buffers
+    pi[3], pi[5], pi[6], pi[8] = H, H // 2, H, 0
     pi.tofile(os.path.join(d, "params_i.bin"))
     # the emulator's own barriers store their (equal) thread count on every use
     (d / "supp").write_text("race:pair_barrier\n")
@@ -97,3 +98,10 @@ def test_free_slots_read_before_they_change(emu_exe, tmp_path, prephase, cuts):
     """The free-slot mask: every lane has read it before a lane stores it."""
     got = reports(emu_exe, tmp_path, 16, prephase, cuts)
     assert not [s for s in got if "beam_apply_hap" in s], got
+
+
+@pytest.mark.parametrize("P,H,cuts", [(16, 8, range(24, 28)), (4, 2, range(30, 34)), (128, 30, range(44, 46))])
+def test_nothing_reported(emu_exe, tmp_path, P, H, cuts):
+    """Small and wide beams (more than 32 paths), a ring as long as the history
+    (whose entry 0 is rescaled twice) and a longer one."""
+    assert reports(emu_exe, tmp_path, P, True, cuts, H) == []
