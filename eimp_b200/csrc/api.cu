@@ -491,10 +491,12 @@ int eimp_imp_prepare_dev(eimp_ctx *ctx, size_t ntargets, const uint64_t *d_phase
     const size_t nsearch = ctx->i_tgthap_n ? ctx->i_ntgthaps : nh;
     if (hapmap) CK(cudaMemsetAsync(ctx->i_nmatch.p, 0, nh * sizeof(int), ctx->stream));
     // up to 2048 haplotypes per launch move a large tree to a global pool
-    // instead of being redone by the retry launch; few haplotypes are searched
-    // in several parts, each of which may
+    // instead of being redone by the retry launch; without set-maximal errors
+    // few haplotypes are searched in several parts, each of which may: up to
+    // eight pools each, where there can be as many parts
+    const size_t parts = setmaxerrors > 0 ? 1 : std::min<size_t>(8, smm_list_max_chunks((int)M));
     const int gslots =
-        ctx->shape_smm_pools ? (int)std::min<size_t>(std::max<size_t>(nsearch, std::min<size_t>(8 * nsearch, 256)), 2048) : 0;
+        ctx->shape_smm_pools ? (int)std::min<size_t>(std::max<size_t>(nsearch, std::min<size_t>(parts * nsearch, 256)), 2048) : 0;
     CK(ctx->i_gpool.reserve((size_t)gslots * smm_gpool_slot_bytes((int)ctx->i_K)));
     CK(ctx->i_gnext.reserve(sizeof(int)));
     CK(cudaMemsetAsync(ctx->i_gnext.p, 0, sizeof(int), ctx->stream));

@@ -65,6 +65,7 @@ cudaError_t launch_smm_list(const uint32_t *compr, int M, int K, const uint64_t 
                             int nhaps, const int32_t *hapmap, int4 *matches, int cap, int *nmatch, uint32_t *status,
                             void *gpool, int gpool_slots, int *gpool_next, cudaStream_t st);
 size_t smm_list_slot_bytes(int K);
+int smm_list_max_chunks(int M);   // parts M sites are searched in, at most
 // refmap (null: identity): panel haplotype of each PBWT haplotype (the
 // reduced reference without the haploid samples' placeholder columns)
 cudaError_t launch_dosage(const int4 *matches, int cap, const int *nmatch, const int32_t *absperm, int K,

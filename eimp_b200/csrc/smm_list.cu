@@ -685,6 +685,9 @@ __global__ void __launch_bounds__(32) smm_list_join_kernel(int M, const int32_t 
 // ---------------------------------------------------------------------------
 size_t smm_list_slot_bytes(int K) { return K <= 65536 ? sizeof(SlList<false, SL_POOL>) : sizeof(SlList<true, SL_POOL>); }
 
+// A chunk is no shorter than 128 sites, about the length of a match.
+int smm_list_max_chunks(int M) { return M / 128 < 1 ? 1 : M / 128 > SL_CHUNKS ? SL_CHUNKS : M / 128; }
+
 struct SlShape { int warps, chunks, group; size_t stage, smem; };
 
 // Chunks, haplotypes per CTA and the ring for a search.  Narrow intervals (at
@@ -710,13 +713,12 @@ static SlShape sl_shape(int M, int K, int nhaps, int cap, int nsm, int lim, int 
     // Chunks for about 12 warps per SM.  Of 1, 4, 8, 12, 16 and 24, with three
     // batches in flight: 400 haplotypes x 2,000 sites 0.50, 0.41, 0.47, 0.40,
     // 0.45, 0.51 ms; 128 x 3,000 1.40, 1.25, 1.02, 1.03, 1.11, 1.52 ms (with
-    // 1,000 haplotypes it is one chunk up to 12, and two are 4 % slower).  No
-    // shorter than 128 sites, about the length of a match: 64 and 256 make
-    // no difference beyond the spread, but longer ones leave warps out.
+    // 1,000 haplotypes it is one chunk up to 12, and two are 4 % slower).  With
+    // at least 64 or 256 sites instead of 128 there is no difference beyond
+    // the spread, but longer ones leave warps out.
     long long chunks = (long long)12 * nsm / nhaps;
-    if (chunks > M / 128) chunks = M / 128;
+    if (chunks > smm_list_max_chunks(M)) chunks = smm_list_max_chunks(M);
     if (chunks > cap / 16) chunks = cap / 16;
-    if (chunks > SL_CHUNKS) chunks = SL_CHUNKS;
     for (f.chunks = (int)chunks; f.chunks > 1; f.chunks--)
         for (f.warps = 1; f.warps <= most; f.warps++) {
             f.smem = head + f.warps * list;
