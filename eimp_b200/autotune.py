@@ -61,22 +61,27 @@ def _time(group, fn, reps: int) -> float:
 
 
 def tune_group(group, reps: int = 2,
-               knobs=("dosage_span", "smm_warps", "smm_tree_pools", "beam_slots_pct")) -> dict:
+               knobs=("dosage_span", "smm_warps", "smm_tree_pools", "beam_slots_pct"), setmaxerrors: int = 0) -> dict:
     """Tunes the knobs of one DensityGroup (eimp_b200/batch.py) on its data;
-    returns {knob: {"chosen": value, "ms": {value: best ms}}}."""
+    returns {knob: {"chosen": value, "ms": {value: best ms}}}.  setmaxerrors:
+    what the group imputes with; without errors the match search does not read
+    smm_warps, which stays as it is and is not timed."""
     group.enqueue()   # a full step first: the phased haplotypes and the reference exist
     group.ctx.synchronize()
     stage = {
         "dosage_span": lambda: group.L.eimp_imp_bunch_dev(group.h, 0, group.Mref, group.d_bits.data_ptr(), group.ldb,
                                                           group.d_dos.data_ptr(), group.Mref),
         "smm_warps": lambda: group.L.eimp_imp_prepare_dev(group.h, group.nt, group.d_ph.data_ptr(),
-                                                          group.d_gt.data_ptr(), 0, 0, 0),
+                                                          group.d_gt.data_ptr(), setmaxerrors, 0, 0),
         "smm_tree_pools": lambda: group.L.eimp_imp_prepare_dev(group.h, group.nt, group.d_ph.data_ptr(),
-                                                               group.d_gt.data_ptr(), 0, 0, 0),
+                                                               group.d_gt.data_ptr(), setmaxerrors, 0, 0),
         "beam_slots_pct": group.phase,
     }
     out = {}
     for k in knobs:
+        if k == "smm_warps" and setmaxerrors <= 0:
+            out[k] = {"chosen": get(group, k), "ms": {}}
+            continue
         times = {}
         for v in KNOBS[k][1]:
             set_shape(group, k, v)
