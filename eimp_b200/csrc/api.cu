@@ -135,8 +135,9 @@ int fail(eimp_ctx *c, int code, const std::string &msg) {
 
 #define LAUNCH(call)                                                                               \
     do {                                                                                           \
+        launched_kernels();   /* what was not counted for a context */                             \
         cudaError_t e_ = (call);                                                                   \
-        ctx->launches++;                                                                           \
+        ctx->launches += launched_kernels();                                                       \
         if (e_ != cudaSuccess) return fail(ctx, EIMP_E_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
@@ -505,7 +506,6 @@ int eimp_imp_prepare_dev(eimp_ctx *ctx, size_t ntargets, const uint64_t *d_phase
                       setmaxerrors, ctx->i_matches.as<int4>(), (int)cap, ctx->i_nmatch.as<int>(),
                       ctx->status.as<uint32_t>(), ctx->shape_smm_warps, gslots ? ctx->i_gpool.p : nullptr, gslots,
                       ctx->i_gnext.as<int>(), ctx->stream));
-    ctx->launches++;   // launch_smm launches twice: the small node pool, then the retry pass
     return 0;
 }
 
@@ -1292,6 +1292,17 @@ size_t eimp_gpu_block_size(const eimp_ctx *ctx) { (void)ctx; return 1024; }
 }  // extern "C"
 
 namespace eimp {
+static thread_local unsigned launch_count = 0;
+cudaError_t launched(int n) {
+    launch_count += (unsigned)n;
+    return cudaGetLastError();
+}
+unsigned launched_kernels() {
+    const unsigned n = launch_count;
+    launch_count = 0;
+    return n;
+}
+
 cudaError_t ensure_dynamic_smem(const void *kernel, size_t bytes) {
     static std::mutex mu;
     static std::map<std::pair<int, const void *>, size_t> limit;   // per device and kernel

@@ -2016,13 +2016,13 @@ cudaError_t launch_beam(const BeamParams &p, int ntgt, int M, const uint8_t *gt,
     cudaError_t e = ensure_dynamic_smem((const void *)beam_kernel, s.smem);
     if (e != cudaSuccess) return e;
     lpt_order_kernel<<<1, 1024, 0, st>>>(nsplits, ntgt, order, skip);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if ((e = launched()) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(workq, 0, sizeof(int), st)) != cudaSuccess) return e;
     beam_kernel<<<slots, 32 * s.warps, s.smem, st>>>(p, al, ntgt, M, gt, monos, splits, nsplits, calls,
                                                               ncalls, cmdiffs, pbwt, count0, rowoff,
                                                               (uint8_t *)arena, arena_bytes, mats, pats, dmat, dpat,
                                                               totalconf, ncallsites, status, skip, order, workq);
-    return cudaGetLastError();
+    return launched();
 }
 
 }  // namespace eimp

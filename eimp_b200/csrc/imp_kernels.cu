@@ -1247,7 +1247,7 @@ cudaError_t launch_refpbwt(const uint64_t *sitemajor, int M, int K, int wN, uint
         auto ck = in_smem ? refpbwt_ckpt_kernel<1> : refpbwt_ckpt_kernel<8>;
         if ((e = ensure_dynamic_smem((const void *)ck, sm)) != cudaSuccess) return e;
         ck<<<1, 1024, sm, st>>>(sitemajor, M, K, wN, absperm, in_smem ? nullptr : scratch, stage ? 1 : 0);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        if ((e = launched()) != cudaSuccess) return e;
     }
     if (M <= 0) return cudaSuccess;
     const size_t sm = refpbwt_fill_smem(K, wN);
@@ -1258,7 +1258,7 @@ cudaError_t launch_refpbwt(const uint64_t *sitemajor, int M, int K, int wN, uint
     const int ck = refpbwt_by_blocks(M, K) ? RP_SUB : RP_CK;
     if ((e = ensure_dynamic_smem((const void *)fill, sm)) != cudaSuccess) return e;
     fill<<<(M + ck - 1) / ck, 1024, sm, st>>>(sitemajor, M, K, wN, compr, absperm, count0);
-    return cudaGetLastError();
+    return launched();
 }
 
 cudaError_t launch_gather_rows(const uint64_t *src, size_t ldsrc, const int64_t *idx, int n, int w, uint64_t *dst,
@@ -1266,7 +1266,7 @@ cudaError_t launch_gather_rows(const uint64_t *src, size_t ldsrc, const int64_t 
     const long tot = (long)n * w;
     if (tot == 0) return cudaSuccess;
     gather_rows_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(src, ldsrc, idx, n, w, dst);
-    return cudaGetLastError();
+    return launched();
 }
 
 cudaError_t launch_transpose(const uint64_t *src, size_t rows, size_t srcw, uint64_t *dst, size_t cols, size_t dstw,
@@ -1283,7 +1283,7 @@ cudaError_t launch_transpose_ld(const uint64_t *src, size_t rows, size_t src_ld,
     if (e != cudaSuccess) return e;
     dim3 grid((unsigned)((dstw * 64 + TR_ROWS - 1) / TR_ROWS), (unsigned)gy);
     transpose_kernel<false><<<grid, TR_ROWS, TR_SMEM, st>>>(src, rows, src_ld, dst, cols, dstw, dst_ld);
-    return cudaGetLastError();
+    return launched();
 }
 
 cudaError_t launch_block_keys(const uint64_t *src, int rows, int src_ld, uint64_t *dst, int cols, size_t dst_ld,
@@ -1293,7 +1293,7 @@ cudaError_t launch_block_keys(const uint64_t *src, int rows, int src_ld, uint64_
     const int ncw = (cols + 63) / 64;
     dim3 grid((unsigned)((rows + TR_ROWS - 1) / TR_ROWS), (unsigned)((ncw + TR_WORDS - 1) / TR_WORDS));
     transpose_kernel<true><<<grid, TR_ROWS, TR_SMEM, st>>>(src, rows, src_ld, dst, cols, (rows + 63) / 64, dst_ld);
-    return cudaGetLastError();
+    return launched();
 }
 
 template <class Smem, class Kern, class... Extra>
@@ -1307,7 +1307,7 @@ static cudaError_t smm_launch(Kern kern, int warps, const uint32_t *compr, const
     const int blocks = (nhaps + warps - 1) / warps;
     kern<<<blocks, warps * 32, sm, st>>>(compr, count0, M, K, phased, wM, gt, nhaps, hapmap, setmaxerrors, matches,
                                         cap, nmatch, status, extra...);
-    return cudaGetLastError();
+    return launched();
 }
 
 size_t smm_gpool_slot_bytes(int K) {
@@ -1396,13 +1396,13 @@ cudaError_t launch_dosage(const int4 *matches, int cap, const int *nmatch, const
     kern<<<(unsigned)blocks, 256, 0, st>>>(matches, cap, nmatch, absperm, K, refmap, hapmajor_full, wMref, sinfo,
                                            phased, wM, gt, M, nhaps, hapmap, mref_begin, nsites, imputeCalls, dos, ldd,
                                            bits, ldb);
-    return cudaGetLastError();
+    return launched();
 }
 
 cudaError_t launch_segmap(const int64_t *typed, int M, int Mref, const float *af, int nrefhaps_total, int32_t *segm,
                           uint8_t *common, int2 *sinfo, cudaStream_t st) {
     segmap_kernel<<<(Mref + 255) / 256, 256, 0, st>>>(typed, M, Mref, af, nrefhaps_total, segm, common, sinfo);
-    return cudaGetLastError();
+    return launched();
 }
 
 }  // namespace eimp

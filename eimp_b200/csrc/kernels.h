@@ -27,6 +27,11 @@ namespace eimp {
 // between another thread's setting and its launch.
 cudaError_t ensure_dynamic_smem(const void *kernel, size_t bytes);
 
+// cudaGetLastError after n kernel launches, which the calling thread's count
+// takes up; launched_kernels: that count, since its last call
+cudaError_t launched(int n = 1);
+unsigned launched_kernels();
+
 
 // ---- imputation (imp_kernels.cu)
 // global scratch launch_refpbwt needs (0: none) for M sites of K haplotypes

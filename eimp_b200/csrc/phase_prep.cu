@@ -260,11 +260,11 @@ cudaError_t launch_besthaps(const uint8_t *gt, int ntgt, int M, const uint64_t *
         dim3 grid((unsigned)((ntgt + tb - 1) / tb),
                   (unsigned)((nhaps + HAM_WARPS * HAM_HPW - 1) / (HAM_WARPS * HAM_HPW)));
         kern<<<grid, 32 * HAM_WARPS, sm, st>>>(gt, ntgt, M, hapmajor, nhaps, wM, nerr_scratch, self0, haploid);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        if ((e = launched()) != cudaSuccess) return e;
     }
     besthaps_kernel<<<ntgt, 512, 0, st>>>(gt, M, hapmajor, nhaps, wM, K, nerr_scratch, besthaps, flags, wN, self0,
                                           haploid);
-    return cudaGetLastError();
+    return launched();
 }
 
 // ---------------------------------------------------------------------------
@@ -438,7 +438,7 @@ cudaError_t launch_monos_calls(const uint8_t *gt, int ntgt, int M, const uint64_
     if (sm > 48 * 1024 && (e = ensure_dynamic_smem((const void *)kern, sm)) != cudaSuccess) return e;
     kern<<<ntgt, many ? 256 : 1024, sm, st>>>(gt, M, hapmajor, wM, besthaps, K, cm, cMmaxsplit, monos, splits, calls,
                                               cmdiffs, nsplits, ncalls, tgt_haploid);
-    return cudaGetLastError();
+    return launched();
 }
 
 // ---------------------------------------------------------------------------
@@ -486,7 +486,7 @@ cudaError_t launch_haploid_phase(const uint8_t *gt, int ntgt, int M, int wM, con
                                  int32_t *ncallsites, uint32_t *status, cudaStream_t st) {
     haploid_phase_kernel<<<ntgt, 256, 0, st>>>(gt, M, wM, tgt_haploid, mats, pats, dmat, dpat, totalconf, ncallsites,
                                                status);
-    return cudaGetLastError();
+    return launched();
 }
 
 // ---------------------------------------------------------------------------
@@ -525,7 +525,7 @@ cudaError_t launch_compact_cols(const uint64_t *src, int rows, int srcw, const i
                                 int dstw, cudaStream_t st) {
     const long n = (long)rows * dstw;
     compact_cols_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(src, rows, srcw, map, ncols, dst, dstw);
-    return cudaGetLastError();
+    return launched();
 }
 
 // ---------------------------------------------------------------------------
@@ -633,7 +633,7 @@ cudaError_t launch_cref(const uint8_t *gt, int ntgt, int M, const uint64_t *hapm
     dim3 grid((unsigned)ntgt, (unsigned)((2 * wK + CREF_WARPS - 1) / CREF_WARPS));
     cref_kernel<<<grid, 32 * CREF_WARPS, sm, st>>>(gt, M, hapmajor, wM, nhaps, besthaps, K, splits, nsplits, rowoff,
                                                    cref, skip);
-    return cudaGetLastError();
+    return launched();
 }
 
 // ---------------------------------------------------------------------------
@@ -832,7 +832,7 @@ static cudaError_t launch_pbwt_w(int sub, const uint64_t *cref, int32_t *count0,
     cudaError_t e = ensure_dynamic_smem((const void *)kern, sm);
     if (e != cudaSuccess) return e;
     kern<<<2 * ntgt, nthreads, sm, st>>>(cref, rowoff, K, pbwt, rowstride, emit_padded, count0, skip);
-    return cudaGetLastError();
+    return launched();
 }
 
 cudaError_t launch_pbwt(const uint64_t *cref, int32_t *count0, const int64_t *rowoff, int ntgt, int K,
@@ -888,7 +888,7 @@ __global__ void __launch_bounds__(1024) rowoff_kernel(const int32_t *__restrict_
 cudaError_t launch_rowoff(const int32_t *nsplits, int ntgt, int64_t *rowoff, int64_t cap, int *skip,
                           uint32_t *status, cudaStream_t st) {
     rowoff_kernel<<<1, 1024, 0, st>>>(nsplits, ntgt, rowoff, cap, skip, status);
-    return cudaGetLastError();
+    return launched();
 }
 
 }  // namespace eimp

@@ -187,14 +187,14 @@ cudaError_t launch_qref_mask(const uint8_t *sec, const int64_t *offs, int nvar, 
     if (nvar <= 0) return cudaSuccess;
     qref_mask_kernel<<<(nvar + 3) / 4, 128, 0, st>>>(sec, offs, nvar, rows, ldr, kept, nkept, nwout, masked, nmasked,
                                                      masked_hap, an_before, an_after, af, out, ldo);
-    return cudaGetLastError();
+    return launched();
 }
 
 cudaError_t launch_qref_decode(const uint8_t *sec, const int64_t *offs, int Mref, int nwords, uint64_t *out,
                                size_t ldw, uint32_t *status, cudaStream_t st) {
     if (Mref <= 0) return cudaSuccess;
     qref_decode_kernel<<<(Mref + 3) / 4, 128, 0, st>>>(sec, offs, Mref, nwords, out, ldw, status);
-    return cudaGetLastError();
+    return launched();
 }
 
 }  // namespace eimp

@@ -466,24 +466,25 @@ cudaError_t launch_refpbwt_blocks(const uint64_t *sitemajor, int M, int K, int w
         if (ranked) rp_order_kernel<false><<<groups, 1024, ro, st>>>(absperm, K, nblocks, group);
         if ((e = ensure_dynamic_smem((const void *)rp_sub_kernel, ro)) != cudaSuccess) return e;
         rp_sub_kernel<<<subs, 1024, ro, st>>>(absperm, M, K);   // a site count past RB_SUB leaves at least one
-        return cudaGetLastError();
+        return launched((ranked ? 2 : 0) + (groups > 1 ? 1 : 0) + 2);
     }
     if ((e = ensure_dynamic_smem((const void *)rp_class_kernel<int32_t>, rc)) != cudaSuccess) return e;
     if (ranked) rp_class_kernel<int32_t><<<ranked, 1024, rc, st>>>(absperm, K, ranked, 0, RB_BITS);
     int width = 1;
     while ((1 << width) < K) width++;
+    const int rank_passes = (width + RW_DIGIT - 1) / RW_DIGIT, site_passes = (RB_SUB + RW_DIGIT - 1) / RW_DIGIT;
     for (int b = 0; b < ranked; b++)
-        for (int p = 0; p < (width + RW_DIGIT - 1) / RW_DIGIT; p++) {
+        for (int p = 0; p < rank_passes; p++) {
             rw_count_kernel<<<RW_CTAS, 512, 0, st>>>(absperm, M, K, b, -1, p);
             rw_place_kernel<<<RW_CTAS, 512, 0, st>>>(absperm, M, K, b, -1, p);
         }
     const dim3 all(RW_CTAS, (unsigned)subs);
     for (int s = 0; s + 1 < RB_SITES / RB_SUB; s++)
-        for (int p = 0; p < (RB_SUB + RW_DIGIT - 1) / RW_DIGIT; p++) {
+        for (int p = 0; p < site_passes; p++) {
             rw_count_kernel<<<all, 512, 0, st>>>(absperm, M, K, 0, s, p);
             rw_place_kernel<<<all, 512, 0, st>>>(absperm, M, K, 0, s, p);
         }
-    return cudaGetLastError();
+    return launched((ranked ? 1 : 0) + 2 * ranked * rank_passes + 2 * (RB_SITES / RB_SUB - 1) * site_passes);
 }
 
 }  // namespace eimp

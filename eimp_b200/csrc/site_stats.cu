@@ -282,7 +282,7 @@ cudaError_t launch_site_stats(const SiteStatsArgs &a, cudaStream_t st) {
     // haploid targets in a separate instantiation: the diploid one keeps its registers
     if (a.haptgt) launch_site_stats_t<true>(a, grid, block, st);
     else launch_site_stats_t<false>(a, grid, block, st);
-    return cudaGetLastError();
+    return launched();
 }
 
 }  // namespace eimp

@@ -756,7 +756,7 @@ static cudaError_t smm_list_launch(const uint32_t *compr, int M, int K, const ui
         static_cast<SlList<WIDE, SL_POOL> *>(gpool), gpool_slots, gpool_next, f.chunks);
     if (f.chunks > 1)
         smm_list_join_kernel<<<nhaps, 32, 0, st>>>(M, hapmap, matches, cap, nmatch, status, f.chunks);
-    return cudaGetLastError();
+    return launched(f.chunks > 1 ? 2 : 1);
 }
 
 cudaError_t launch_smm_list(const uint32_t *compr, int M, int K, const uint64_t *phased, int wM, const uint8_t *gt,
