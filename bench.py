@@ -771,7 +771,7 @@ def main():
     roofline = {"kernel": "beam_kernel", "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "peak_source": peak_kind, "traffic": traffic,
                 "algorithmic_bytes_per_launch": st_by["beam"], "avg_launch_ms": beam_ms,
-                "note": "latency-bound: one warp per target walks the beam sequentially; all batches of all groups",
+                "note": "latency-bound: a target's beam is a serial chain of steps, one CTA each; all batches of all groups",
                 "step": {"algorithmic_bytes": step_bytes, "ms": ms_per_step,
                          "achieved_gbs": step_bytes / (ms_per_step / 1e3) / 1e9,
                          "frac": step_bytes / (ms_per_step / 1e3) / 1e9 / peak},

@@ -66,8 +66,8 @@ __device__ void block_exscan(int *a, int n, int *warpbuf, int *total) {
 // from its checkpoint and steps site by site, writing every prefix array,
 // compressed row and zero count of its interval.
 // ---------------------------------------------------------------------------
-constexpr int RP_CK = 64;     // sites between checkpoint orders
-constexpr int RP_SUB = 16;    // sites between the orders of refpbwt_blocks.cu
+constexpr int RP_CK = REFPBWT_BLOCK;    // sites between checkpoint orders
+constexpr int RP_SUB = REFPBWT_SUB;     // sites between the orders of refpbwt_blocks.cu
 constexpr int RP_BITS = 5;    // sites per step of the checkpoint pass: 32 buckets, one per lane
 // rounds of 32 positions whose loads are issued together: 8 with the orders
 // in global memory (their latency overlapped), 1 in shared memory (fewer
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(1024, 1) refpbwt_ckpt_kernel(const uint64_t *_
 }
 
 // Fill pass: CTA c covers sites [c*CK, min(M, (c+1)*CK)); the order before its
-// first site is there (from the checkpoint pass, or every RB_SUB sites from
+// first site is there (from the checkpoint pass, or every RP_SUB sites from
 // refpbwt_blocks.cu).  Per site: the bits in prefix
 // order (one ballot per 32 positions), the zeros per 32-position word and
 // their exclusive scan give the compressed row [data, cumulative zeros] and

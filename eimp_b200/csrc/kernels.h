@@ -38,10 +38,14 @@ unsigned launched_kernels();
 size_t refpbwt_scratch_bytes(int M, int K, int wN);
 cudaError_t launch_refpbwt(const uint64_t *sitemajor, int M, int K, int wN, uint32_t *compr, int32_t *absperm,
                            int32_t *count0, int32_t *scratch, cudaStream_t st);
-// the checkpoint orders by blocks of 64 sites (refpbwt_blocks.cu) and where they are used
+// sites between the orders of the one-CTA walk, which are the blocks of
+// refpbwt_blocks.cu, and between the orders of these: the fill pass starts
+// from each
+constexpr int REFPBWT_BLOCK = 64, REFPBWT_SUB = 16;
+// the orders by blocks of sites (refpbwt_blocks.cu) and where they are used
 bool refpbwt_by_blocks(int M, int K);
 cudaError_t launch_refpbwt_blocks(const uint64_t *sitemajor, int M, int K, int wN, int32_t *absperm, cudaStream_t st);
-// word b * dst_ld + c of dst = bits of column c in src rows 64b .. 64b+63 (rows a multiple of 64)
+// word b * dst_ld + c of dst = bits of column c in src rows 64b .. 64b+63, zeros past the last row
 cudaError_t launch_block_keys(const uint64_t *src, int rows, int src_ld, uint64_t *dst, int cols, size_t dst_ld,
                               cudaStream_t st);
 // dst row c (dstw words) = column c of the bit matrix src, zeros past its last row

@@ -6,8 +6,9 @@
 // (PBWT.cpp:207-285 one site at a time).  Of a block of sites only the ranking
 // of its allele patterns matters, and that is the same whatever the order
 // before it: so
-//  * rp_keys_kernel   (imp_kernels.cu) gives every haplotype its 64 alleles of
-//                     a block as one number, the last site its highest bit;
+//  * launch_block_keys (a transpose, imp_kernels.cu) gives every haplotype its 64
+//                     alleles of a block as one number, the last site its
+//                     highest bit;
 //  * rp_class_kernel  replaces them by their dense rank, a CTA per block: the
 //                     haplotypes of a block share few patterns, so a rank has
 //                     ten bits or so instead of 64.  A second launch
@@ -22,7 +23,7 @@
 //                     shared memory;
 //  * rp_sub_kernel (or the same passes over all blocks at once) adds the orders
 //                     every RB_SUB sites inside the blocks, from which
-//                     refpbwt_fill_kernel's CTAs write the rest.
+//                     refpbwt_fill_sub_kernel's CTAs write the rest.
 // With the group size near the square root of the number of blocks the serial
 // chain is two square roots of it long, a few counting-sort passes each, instead
 // of 13 passes per block (refpbwt_ckpt_kernel).
@@ -36,10 +37,10 @@
 
 namespace eimp {
 
-constexpr int RB_SITES = 64;    // sites of a block: the fill pass's checkpoint distance
+constexpr int RB_SITES = REFPBWT_BLOCK;   // sites of a block
 constexpr int RB_BITS = 20;     // pattern bits ranked at a time (a bitmap of 128 KB)
 constexpr int RB_DIGIT = 8;     // sort digit, at most
-constexpr int RB_SUB = 16;      // sites between the orders the fill pass starts from
+constexpr int RB_SUB = REFPBWT_SUB;       // sites between the orders the fill pass starts from
 constexpr int RB_HIST = 32 * ((1 << RB_DIGIT) + 1);   // digit counts, a row per warp (odd stride: a warp's digits in different banks)
 
 // rows of a block's prefix arrays that hold its scratch
@@ -452,7 +453,8 @@ cudaError_t launch_refpbwt_blocks(const uint64_t *sitemajor, int M, int K, int w
                                st)) != cudaSuccess)
         return e;
     const size_t rc = rc_smem_bytes(RB_BITS), ro = ro_smem_bytes(K);
-    // orders in one SM's shared memory (36,000 haplotypes on a B200), or passes over the GPU
+    // orders in one SM's shared memory (6 bytes a haplotype beside 33 KB of counts:
+    // 33,237 haplotypes on a B200), or passes over the GPU
     if (ro <= (size_t)lim) {
         int group = 2;
         while (group * group < nblocks) group++;

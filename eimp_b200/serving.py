@@ -15,8 +15,9 @@ phased haplotypes and imputed dosages.
   ``max_batch_targets`` targets) and into the device-memory budget, whatever
   their sizes; the requests that arrive meanwhile wait for the next free
   slot.  Results are split back per request.  Per-target work is independent
-  (one warp per target in phasing, one per target haplotype in imputation),
-  so a request's result does not depend on what it was batched with.
+  (one CTA per target in phasing, a warp or several per target haplotype in
+  imputation), so a request's result does not depend on what it was batched
+  with.
 * **Admission by device memory.**  Every launch reserves an estimate of its
   device bytes (``bytes_per_target`` x its targets) against ``mem_budget``;
   a launch waits until the reservations in flight leave room for it.  A
