@@ -1950,9 +1950,10 @@ __global__ void __launch_bounds__(BEAM_SM_CTAS * 32 * BEAM_WARPS, 1) beam_kernel
 // most BEAM_SM_CTAS.  The shared memory that is left becomes haplotype-path slots:
 // all of it with a target or less per SM, a BEAM_SM_CTAS-th with more -- a second
 // context's beams then find room beside the last targets of the first (192
-// targets of 32,000 sites, three contexts in turn: 57.5 -> 45.5 ms a pass), and
-// slots that go to the arena for it cost little (1,000 targets of 5,000 sites,
-// one CTA per SM: 107 ms with all slots in shared memory, 112 with 12).
+// targets of 32,000 sites, three contexts in turn: 57.5 -> 45.5 ms a pass; the
+// price is a single context's pass, 61.8 -> 63.0 ms), and slots that go to the
+// arena for it cost little (1,000 targets of 5,000 sites, one CTA per SM: 107 ms
+// with all slots in shared memory, 112 with 12).
 struct BeamShape { int warps, ctas; size_t smem; };
 
 static size_t beam_smem(const BeamParams &p, const ArenaLayout &al, int warps) {
