@@ -631,11 +631,12 @@ __global__ void __launch_bounds__((SL_WARPS + 1) * 32) smm_list_kernel(
 // -- and accepted or refused there as a whole -- when a chunk outgrew its list
 // or its part of the buffer, when the lists of the chunks that share a site
 // could make one larger than the most a list may hold, or when the buffer
-// would have been too small on the way.  The retry launch holds large lists in
-// shared memory, so it also beats this kernel searching them again in one piece:
-// 16 and 200 haplotype pairs x 3,000 sites of 20,000 haplotypes, half the
-// genotypes of 75 sites missing, 1.48 and 14.7 ms against 3.87 and 15.8 (the
-// general kernel alone 19.2 and 36.7; nothing missing in bunches 0.45 and 1.7).
+// would have been too small on the way.  Searching those with this kernel in one
+// piece first, a pool for each, is no better throughout: 16, 64 and 200
+// haplotype pairs x 3,000 sites of 20,000 haplotypes, half the genotypes of 75
+// sites missing, 1.5, 13.9 and 14.7 ms without, 3.9, 11.5 and 15.8 with it (the
+// general kernel alone 19, 33 and 37; without missing genotypes in bunches
+// 0.45, 0.72 and 1.7).
 __global__ void __launch_bounds__(32) smm_list_join_kernel(int M, const int32_t *__restrict__ hapmap,
                                                            int4 *__restrict__ matches, int cap,
                                                            int *__restrict__ nmatch, uint32_t *__restrict__ status,
